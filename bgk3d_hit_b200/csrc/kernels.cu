@@ -36,11 +36,11 @@ __device__ __forceinline__ __half ldg(const __half* p) { return __ldg(p); }
 template <class V>
 __device__ __forceinline__ V moments(const V (&x)[Q], V& vx, V& vy, V& vz) {
   using N = Num<V>;
-  const V uno = N::c(1.0), cte1 = N::c(1.0);
+  const V cte1 = N::c(1.0);
   V rho = x[0] + x[1] + x[2] + x[3] + x[4] + x[5] + x[6] + x[7]
         + x[8] + x[9] + x[10] + x[11] + x[12] + x[13] + x[14] + x[15]
         + x[16] + x[17] + x[18] + cte1;
-  V rhoinv = uno / rho;
+  V rhoinv = ercp(rho);
   vx = (x[0] + x[1] + x[2] + x[3] + x[4] - x[9] - x[10] - x[11] - x[12] - x[13]) * rhoinv;
   vy = (x[2] + x[6] + x[7] + x[8] + x[11] - x[0] - x[9] - x[15] - x[16] - x[17]) * rhoinv;
   vz = (x[3] + x[5] + x[6] + x[12] + x[17] - x[1] - x[8] - x[10] - x[14] - x[15]) * rhoinv;
