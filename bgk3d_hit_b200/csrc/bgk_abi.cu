@@ -42,11 +42,13 @@ int cuda_fail(cudaError_t e, const char* what) {
 // 64..256-byte boundary; populations start on 256-element boundaries.
 constexpr int ROW_ALIGN = 32;
 constexpr long long POP_ALIGN = 256;
-// Staging for host velocity input: this many cells per chunk (whole planes).
-// Cells per chunk of a velocity-field upload from host memory: two staging
-// sets of three such chunks (96 MB) let the copy of one chunk run beside the
-// initialisation kernel of the previous one.
-constexpr long long INIT_CHUNK_CELLS = 1LL << 21;
+// Cells per chunk (whole planes) of a velocity field that goes to or comes
+// from host memory: two staging sets of three such chunks (96 MB) let the copy
+// of one chunk run beside the kernel of its neighbour.
+constexpr long long VEL_CHUNK_CELLS = 1LL << 21;
+// Staging for populations on their way to or from host memory: as many of them
+// per kernel and copy as fit this many bytes (at least one).
+constexpr size_t POP_STAGE_BYTES = 64u << 20;
 
 }  // namespace
 
@@ -75,17 +77,17 @@ struct bgk_ctx {
   long long step = 0;
   double omega = 0.0, scale = 1.0;
   double* partials = nullptr;
-  double* totals = nullptr;
-  double* h_tot = nullptr;  // pinned
+  double* h_tot = nullptr;  // pinned: ND totals, zj of the last cell, error flag
   unsigned int* d_max = nullptr;
   int* d_err = nullptr;     // set on the device when a pipelined kernel's wait ran out
   int* h_err = nullptr;     // pinned copy
   void* vel = nullptr;
   void* stage = nullptr;
   size_t stage_bytes = 0;
-  // host upload pipeline: copy stream, staging set filled / free again
+  // host transfer pipelines: copy stream, staging set filled / free again
   cudaStream_t st_copy = nullptr;
   cudaEvent_t ev_full[2] = {nullptr, nullptr}, ev_free[2] = {nullptr, nullptr};
+  cudaEvent_t ev_in = nullptr;  // the default stream's work, for device arrays of the caller
   long long launches = 0;
   long long dev_bytes = 0;
   void* fft_buf = nullptr;
@@ -167,6 +169,20 @@ int ensure_stage(bgk_ctx* c, size_t bytes) {
   return BGK_OK;
 }
 
+// Copy stream and events of the host transfer pipelines. Nothing queued on the
+// context's stream before this call may still use a staging set when the first
+// transfer of the pipeline reaches it.
+int begin_transfer(bgk_ctx* c) {
+  if (!c->st_copy) CK(cudaStreamCreateWithFlags(&c->st_copy, cudaStreamNonBlocking));
+  for (int b = 0; b < 2; ++b) {
+    if (!c->ev_full[b]) CK(cudaEventCreateWithFlags(&c->ev_full[b], cudaEventDisableTiming));
+    if (!c->ev_free[b]) CK(cudaEventCreateWithFlags(&c->ev_free[b], cudaEventDisableTiming));
+  }
+  CK(cudaEventRecord(c->ev_free[0], c->st));
+  CK(cudaEventRecord(c->ev_free[1], c->st));
+  return BGK_OK;
+}
+
 int ensure_vel(bgk_ctx* c) {
   if (c->vel) return BGK_OK;
   return dev_alloc(c, &c->vel, 3 * (size_t)ncell(c) * rsize(c), "velocity field");
@@ -227,21 +243,45 @@ int set_scale_from_max(bgk_ctx* c) {
 
 int init_layout(const bgk_ctx* c) { return c->scheme == BGK_AA ? LAY_AAE : LAY_TWO; }
 
-// Synchronises the stream and reports a bounded wait of a pipelined kernel
-// that ran out (the step it belonged to did not complete).
+// A bounded wait of a pipelined kernel ran out: the step it belonged to did not
+// complete.
+int step_failed() {
+  set_err("a stream-collide step gave up waiting for its row copies; populations are invalid");
+  return BGK_ERR_CUDA;
+}
+
+// Synchronises the stream and reports such a step.
 int sync_and_check(bgk_ctx* c) {
   CK(cudaMemcpyAsync(c->h_err, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->st));
   CK(cudaStreamSynchronize(c->st));
-  if (*c->h_err) {
-    set_err("a stream-collide step gave up waiting for its row copies; populations are invalid");
-    return BGK_ERR_CUDA;
+  return *c->h_err ? step_failed() : BGK_OK;
+}
+
+// Orders the context's stream behind the default stream, where callers usually
+// make the device arrays that they hand over. Left out while a capture forbids
+// touching the default stream.
+int after_default_stream(bgk_ctx* c) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(cudaStreamLegacy, &cap) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return BGK_OK;
   }
+  if (cap != cudaStreamCaptureStatusNone) return BGK_OK;
+  if (!c->ev_in) CK(cudaEventCreateWithFlags(&c->ev_in, cudaEventDisableTiming));
+  CK(cudaEventRecord(c->ev_in, cudaStreamLegacy));
+  CK(cudaStreamWaitEvent(c->st, c->ev_in, 0));
   return BGK_OK;
+}
+
+// Planes per chunk of a velocity field's host transfer.
+int chunk_planes(const bgk_ctx* c) {
+  const long long nk = VEL_CHUNK_CELLS / ((long long)c->g.nx * c->g.ny);
+  return nk < 1 ? 1 : nk > c->g.nz ? c->g.nz : (int)nk;
 }
 
 // Equilibrium initial condition from a velocity field: host arrays go
 // through a staging buffer in chunks of whole planes; device arrays (on the
-// context's device) are read in place, chunk by chunk in the same order.
+// context's device) are read in place by one launch.
 int init_velocity_impl(bgk_ctx* c, const double* u, const double* v, const double* w, double rho, bool on_device) {
   int rc = check_ctx(c);
   if (rc) return rc;
@@ -263,26 +303,17 @@ int init_velocity_impl(bgk_ctx* c, const double* u, const double* v, const doubl
         return BGK_ERR_INVALID;
       }
     }
+    if ((rc = after_default_stream(c))) return rc;
   }
   const long long plane = (long long)c->g.nx * c->g.ny;
-  int nk = (int)(INIT_CHUNK_CELLS / plane);
-  if (nk < 1) nk = 1;
-  if (nk > c->g.nz) nk = c->g.nz;
+  const int nk = on_device ? c->g.nz : chunk_planes(c);
   const size_t chunk = (size_t)plane * nk;
   double *su = nullptr, *sv = nullptr, *sw = nullptr;
   if (!on_device) {
     // two staging sets of three chunks; the copies run on their own stream
     rc = ensure_stage(c, 2 * 3 * chunk * sizeof(double));
     if (rc) return rc;
-    if (!c->st_copy) CK(cudaStreamCreateWithFlags(&c->st_copy, cudaStreamNonBlocking));
-    for (int b = 0; b < 2; ++b) {
-      if (!c->ev_full[b]) CK(cudaEventCreateWithFlags(&c->ev_full[b], cudaEventDisableTiming));
-      if (!c->ev_free[b]) CK(cudaEventCreateWithFlags(&c->ev_free[b], cudaEventDisableTiming));
-    }
-    // nothing queued on the context's stream before this call may still
-    // read a staging set when the first copies land
-    CK(cudaEventRecord(c->ev_free[0], c->st));
-    CK(cudaEventRecord(c->ev_free[1], c->st));
+    if ((rc = begin_transfer(c))) return rc;
   }
   const int lay = init_layout(c);
   const bool measure = c->form == FORM_F16 && c->p.fp16_scale == 0.0;
@@ -377,16 +408,17 @@ int compute_diag(bgk_ctx* c, int itime, bgk_diag* out, int want_extras) {
     CK(launch_enstrophy(c->A, c->vel, c->partials, c->st));
     c->launches++;
   }
-  CK(launch_finalize(c->partials, c->totals, c->st));
+  // the totals and the error flag go straight to pinned host memory: no copies
+  // behind the kernels (two of them were a tenth of a 32^3 box's diagnostics)
+  CK(launch_finalize(c->partials, c->h_tot, c->st, c->d_err));
   c->launches++;
   const bool faithful = c->p.mode == BGK_FAITHFUL;
   if (faithful) {
-    CK(launch_last_zj(c->A, c->lay, c->scale, c->totals + ND, c->st));
+    CK(launch_last_zj(c->A, c->lay, c->scale, c->h_tot + ND, c->st));
     c->launches++;
   }
-  CK(cudaMemcpyAsync(c->h_tot, c->totals, (ND + 1) * sizeof(double), cudaMemcpyDeviceToHost, c->st));
-  int rc = sync_and_check(c);
-  if (rc) return rc;
+  CK(cudaStreamSynchronize(c->st));
+  if (c->h_tot[ND + 1] != 0.0) return step_failed();
   const double* t = c->h_tot;
   // a z-slab returns its contribution to the global means
   const double N = global_cells(c);
@@ -423,6 +455,73 @@ int compute_diag(bgk_ctx* c, int itime, bgk_diag* out, int want_extras) {
     return BGK_ERR_NONFINITE;
   }
   return BGK_OK;
+}
+
+// Whether the populations are dense in the reference's order: no row padding,
+// and each population of a cell in the cell's own place.
+bool dense_rows(const bgk_ctx* c) { return c->g.nx == c->g.sx && c->lay != LAY_AAN; }
+
+// Populations straight between lattice a and a host array (out: to it, in: from
+// it), for a box of dense rows. Populations that follow each other on both sides
+// go in one copy (two copies for a whole two-lattice box whose cell count is a
+// multiple of 256; one kernel and one copy per population before).
+int copy_direct(bgk_ctx* c, void* out, const void* in, int lay) {
+  const size_t pop = (size_t)ncell(c) * c->es;
+  auto at = [&](int q) { return (char*)c->A.p[lay == LAY_AAE ? oppq(q) : q]; };
+  for (int q = 0; q < Q;) {
+    int m = 1;
+    while (q + m < Q && at(q + m) == at(q) + m * pop) ++m;
+    if (out) CK(cudaMemcpyAsync((char*)out + q * pop, at(q), m * pop, cudaMemcpyDeviceToHost, c->st));
+    else CK(cudaMemcpyAsync(at(q), (const char*)in + q * pop, m * pop, cudaMemcpyHostToDevice, c->st));
+    q += m;
+  }
+  return out ? sync_and_check(c) : BGK_OK;
+}
+
+// Staging for populations of pop bytes each; *nq: how many it holds at a time.
+int ensure_pop_stage(bgk_ctx* c, size_t pop, int* nq) {
+  size_t want = (size_t)Q * pop < POP_STAGE_BYTES ? (size_t)Q * pop : POP_STAGE_BYTES;
+  if (want < pop) want = pop;
+  if (want < (size_t)ncell(c) * 8) want = (size_t)ncell(c) * 8;
+  const int rc = ensure_stage(c, want);
+  if (rc) return rc;
+  const size_t m = c->stage_bytes / pop;
+  *nq = m > (size_t)Q ? Q : (int)m;
+  return BGK_OK;
+}
+
+// All populations to host memory through the export kernel, elem bytes per
+// value (stored: in the stored type, else double deviations). Where the
+// staging holds several populations but not all, its halves alternate and the
+// copies run beside the next kernel.
+int export_to_host(bgk_ctx* c, char* host, size_t elem, bool stored) {
+  const size_t pop = (size_t)ncell(c) * elem;
+  int nq = 0;
+  int rc = ensure_pop_stage(c, pop, &nq);
+  if (rc) return rc;
+  const bool piped = nq < Q && nq > 1;
+  if (piped) nq /= 2;
+  if (piped && (rc = begin_transfer(c))) return rc;
+  const cudaStream_t sc = piped ? c->st_copy : c->st;
+  int set = 0;
+  for (int q = 0; q < Q; q += nq) {
+    const int m = q + nq < Q ? nq : Q - q;
+    char* s = (char*)c->stage + (size_t)set * nq * pop;
+    if (piped) CK(cudaStreamWaitEvent(c->st, c->ev_free[set], 0));
+    CK(launch_export(c->A, c->lay, q, m, stored ? s : nullptr, stored ? nullptr : (double*)s, c->scale, c->st));
+    c->launches++;
+    if (piped) {
+      CK(cudaEventRecord(c->ev_full[set], c->st));
+      CK(cudaStreamWaitEvent(sc, c->ev_full[set], 0));
+    }
+    CK(cudaMemcpyAsync(host + q * pop, s, m * pop, cudaMemcpyDeviceToHost, sc));
+    if (piped) {
+      CK(cudaEventRecord(c->ev_free[set], sc));
+      set ^= 1;
+    }
+  }
+  if (piped) CK(cudaStreamSynchronize(sc));
+  return sync_and_check(c);
 }
 
 }  // namespace
@@ -576,8 +675,6 @@ int bgk_create(const bgk_params* p, bgk_ctx** out) {
   }
   rc = dev_alloc(c, (void**)&c->partials, (size_t)DIAG_BLOCKS * ND * 2 * sizeof(double), "diagnostic partials");
   if (rc) return fail(rc);
-  rc = dev_alloc(c, (void**)&c->totals, (ND + 1) * sizeof(double), "diagnostic totals");
-  if (rc) return fail(rc);
   rc = dev_alloc(c, (void**)&c->d_max, sizeof(unsigned int), "scale probe");
   if (rc) return fail(rc);
   rc = dev_alloc(c, (void**)&c->d_err, sizeof(int), "error flag");
@@ -587,7 +684,7 @@ int bgk_create(const bgk_params* p, bgk_ctx** out) {
   e = cudaMallocHost((void**)&c->h_err, sizeof(int));
   if (e != cudaSuccess) return fail(cuda_fail(e, "cudaMallocHost"));
   c->A.err = c->B.err = c->d_err;
-  e = cudaMallocHost((void**)&c->h_tot, (ND + 1) * sizeof(double));
+  e = cudaMallocHost((void**)&c->h_tot, (ND + 2) * sizeof(double));
   if (e != cudaSuccess) return fail(cuda_fail(e, "cudaMallocHost"));
   if (c->slab) {
     c->plane_elems = (sx * p->ly + POP_ALIGN - 1) / POP_ALIGN * POP_ALIGN;
@@ -617,7 +714,6 @@ int bgk_destroy(bgk_ctx* c) {
   cudaFree(c->memA);
   cudaFree(c->memB);
   cudaFree(c->partials);
-  cudaFree(c->totals);
   cudaFree(c->d_max);
   cudaFree(c->d_err);
   if (c->h_err) cudaFreeHost(c->h_err);
@@ -634,6 +730,7 @@ int bgk_destroy(bgk_ctx* c) {
   cudaFree(c->adj_tot);
   if (c->h_tot) cudaFreeHost(c->h_tot);
   if (c->mark) cudaEventDestroy(c->mark);
+  if (c->ev_in) cudaEventDestroy(c->ev_in);
   if (c->ev_fork) cudaEventDestroy(c->ev_fork);
   if (c->ev_join) cudaEventDestroy(c->ev_join);
   if (c->ev_edge0) cudaEventDestroy(c->ev_edge0);
@@ -914,31 +1011,16 @@ int bgk_get_populations(bgk_ctx* c, void* host) {
   if (rc) return rc;
   if (!host) return BGK_ERR_INVALID;
   CK(cudaSetDevice(c->p.device));
-  const size_t n = (size_t)ncell(c);
-  rc = ensure_stage(c, n * 8);
-  if (rc) return rc;
-  for (int q = 0; q < Q; ++q) {
-    CK(launch_export(c->A, c->lay, q, c->stage, nullptr, c->scale, c->st));
-    c->launches++;
-    CK(cudaMemcpyAsync((char*)host + q * n * c->es, c->stage, n * c->es, cudaMemcpyDeviceToHost, c->st));
-  }
-  return sync_and_check(c);
+  return dense_rows(c) ? copy_direct(c, host, nullptr, c->lay) : export_to_host(c, (char*)host, c->es, true);
 }
 
 int bgk_get_deviations(bgk_ctx* c, double* host) {
   int rc = check_init(c);
   if (rc) return rc;
   if (!host) return BGK_ERR_INVALID;
+  if (c->form == FORM_F64) return bgk_get_populations(c, host);  // stored as deviations
   CK(cudaSetDevice(c->p.device));
-  const size_t n = (size_t)ncell(c);
-  rc = ensure_stage(c, n * 8);
-  if (rc) return rc;
-  for (int q = 0; q < Q; ++q) {
-    CK(launch_export(c->A, c->lay, q, nullptr, (double*)c->stage, c->scale, c->st));
-    c->launches++;
-    CK(cudaMemcpyAsync(host + q * n, c->stage, n * 8, cudaMemcpyDeviceToHost, c->st));
-  }
-  return sync_and_check(c);
+  return export_to_host(c, (char*)host, 8, false);
 }
 
 int bgk_put_populations(bgk_ctx* c, const void* host) {
@@ -946,14 +1028,21 @@ int bgk_put_populations(bgk_ctx* c, const void* host) {
   if (rc) return rc;
   if (!host) return BGK_ERR_INVALID;
   CK(cudaSetDevice(c->p.device));
-  const size_t n = (size_t)ncell(c);
-  rc = ensure_stage(c, n * 8);
-  if (rc) return rc;
+  const size_t pop = (size_t)ncell(c) * c->es;
   const int lay = c->initialized ? c->lay : init_layout(c);
-  for (int q = 0; q < Q; ++q) {
-    CK(cudaMemcpyAsync(c->stage, (const char*)host + q * n * c->es, n * c->es, cudaMemcpyHostToDevice, c->st));
-    CK(launch_import(c->A, lay, q, c->stage, c->st));
-    c->launches++;
+  if (c->g.nx == c->g.sx && lay != LAY_AAN) {
+    rc = copy_direct(c, nullptr, host, lay);
+    if (rc) return rc;
+  } else {
+    int nq = 0;
+    rc = ensure_pop_stage(c, pop, &nq);
+    if (rc) return rc;
+    for (int q = 0; q < Q; q += nq) {
+      const int m = q + nq < Q ? nq : Q - q;
+      CK(cudaMemcpyAsync(c->stage, (const char*)host + q * pop, m * pop, cudaMemcpyHostToDevice, c->st));
+      CK(launch_import(c->A, lay, q, m, c->stage, c->st));
+      c->launches++;
+    }
   }
   CK(cudaMemsetAsync(c->d_err, 0, sizeof(int), c->st));
   CK(cudaStreamSynchronize(c->st));
@@ -970,24 +1059,33 @@ int bgk_get_velocity(bgk_ctx* c, double* u, double* v, double* w) {
   if (rc) return rc;
   if (!u || !v || !w) return BGK_ERR_INVALID;
   CK(cudaSetDevice(c->p.device));
-  rc = ensure_vel(c);
+  // chunks of planes through two staging sets: the copies of one chunk run
+  // beside the kernel of the next
+  const int nk = chunk_planes(c);
+  const size_t plane = (size_t)c->g.nx * c->g.ny, chunk = plane * nk;
+  rc = ensure_stage(c, 2 * 3 * chunk * sizeof(double));
   if (rc) return rc;
-  CK(launch_diag(c->A, c->lay, c->p.svisc, c->omega, c->scale, c->partials, c->vel, c->st));
-  c->launches++;
-  const size_t n = (size_t)ncell(c);
+  const bool piped = nk < c->g.nz;
+  if (piped && (rc = begin_transfer(c))) return rc;
+  const cudaStream_t sc = piped ? c->st_copy : c->st;
   double* dst[3] = {u, v, w};
-  if (c->form == FORM_F64) {
-    for (int d = 0; d < 3; ++d)
-      CK(cudaMemcpyAsync(dst[d], (double*)c->vel + d * n, n * 8, cudaMemcpyDeviceToHost, c->st));
-    CK(cudaStreamSynchronize(c->st));
-  } else {
-    std::vector<float> tmp(n);
-    for (int d = 0; d < 3; ++d) {
-      CK(cudaMemcpyAsync(tmp.data(), (float*)c->vel + d * n, n * 4, cudaMemcpyDeviceToHost, c->st));
-      CK(cudaStreamSynchronize(c->st));
-      for (size_t s = 0; s < n; ++s) dst[d][s] = (double)tmp[s];
+  int set = 0;
+  for (int k0 = 0; k0 < c->g.nz; k0 += nk, set ^= 1) {
+    const int nkk = k0 + nk <= c->g.nz ? nk : c->g.nz - k0;
+    double* s = (double*)c->stage + (size_t)set * 3 * chunk;
+    if (piped) CK(cudaStreamWaitEvent(c->st, c->ev_free[set], 0));
+    CK(launch_velocity(c->A, c->lay, c->scale, s, true, k0, nkk, c->st));
+    c->launches++;
+    if (piped) {
+      CK(cudaEventRecord(c->ev_full[set], c->st));
+      CK(cudaStreamWaitEvent(sc, c->ev_full[set], 0));
     }
+    for (int d = 0; d < 3; ++d)
+      CK(cudaMemcpyAsync(dst[d] + plane * k0, s + d * plane * nkk, plane * nkk * 8, cudaMemcpyDeviceToHost, sc));
+    if (piped) CK(cudaEventRecord(c->ev_free[set], sc));
   }
+  if (piped) CK(cudaStreamSynchronize(sc));
+  CK(cudaStreamSynchronize(c->st));
   return BGK_OK;
 }
 
@@ -1005,7 +1103,7 @@ int bgk_spectrum(bgk_ctx* c, int nbins, double* ek) {
   CK(cudaSetDevice(c->p.device));
   rc = ensure_vel(c);
   if (rc) return rc;
-  CK(launch_diag(c->A, c->lay, c->p.svisc, c->omega, c->scale, c->partials, c->vel, c->st));
+  CK(launch_velocity(c->A, c->lay, c->scale, c->vel, false, 0, c->g.nz, c->st));
   c->launches++;
   const int nx = c->g.nx, ny = c->g.ny, nz = c->g.nz;
   const size_t cplx = (size_t)nz * ny * (nx / 2 + 1);
@@ -1099,7 +1197,7 @@ int bgk_save(bgk_ctx* c, const char* path) {
   if (rc) return rc;
   std::vector<char> host(n * c->es);
   for (int q = 0; q < Q; ++q) {
-    CK(launch_export(c->A, c->lay, q, c->stage, nullptr, c->scale, c->st));
+    CK(launch_export(c->A, c->lay, q, 1, c->stage, nullptr, c->scale, c->st));
     c->launches++;
     CK(cudaMemcpyAsync(host.data(), c->stage, n * c->es, cudaMemcpyDeviceToHost, c->st));
     rc = sync_and_check(c);
@@ -1146,7 +1244,7 @@ int bgk_load(bgk_ctx* c, const char* path) {
       return BGK_ERR_INVALID;
     }
     CK(cudaMemcpyAsync(c->stage, host.data(), n * c->es, cudaMemcpyHostToDevice, c->st));
-    CK(launch_import(c->A, lay, q, c->stage, c->st));
+    CK(launch_import(c->A, lay, q, 1, c->stage, c->st));
     c->launches++;
     CK(cudaStreamSynchronize(c->st));
   }

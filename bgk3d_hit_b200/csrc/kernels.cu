@@ -20,6 +20,9 @@
 //                per-block partials
 //   k_enstrophy  0.5|curl u|^2 from the local velocity field
 //   k_shift3     shift-only stencil of SRC/do_somethingGPU.F90:37-100
+#include <algorithm>
+#include <cmath>
+
 #include "kernels.h"
 #include "reduce.cuh"
 #include "vec.cuh"
@@ -994,6 +997,42 @@ __global__ void k_halo_prime(Pops<const S> a, Geo g, Halo<S> h) {
   if (threadIdx.x == 0) __threadfence_system();
 }
 
+// ------------------------------------------------------------ row units
+// Rows of a box as units of 32 cells, one per warp: the decode is two 32-bit
+// divisions per warp and unit, and every neighbour offset of a lane is a sum of
+// one of three x, row and plane offsets. (With 64-bit divisions and wraps per
+// access the diagnostics took 750 us in FP32 and FP16 at 256^3, against 196 and
+// 98 us for their bytes at the copy rate: bound by index arithmetic.)
+struct Units {
+  unsigned per_row, per_plane, n;
+  __host__ __device__ explicit Units(int nx, int ny, int nz)
+      : per_row((nx + 31) / 32), per_plane(per_row * ny), n(per_plane * nz) {}
+  __device__ void decode(unsigned u, int& i, int& j, int& k) const {
+    const unsigned z = u / per_plane, r = u - z * per_plane, y = r / per_row;
+    k = (int)z;
+    j = (int)y;
+    i = (int)((r - y * per_row) * 32 + (threadIdx.x & 31));
+  }
+};
+
+// Offsets of the cells around (i, j, k): off(dx, dy, dz), each -1, 0 or 1.
+struct Around {
+  int x[3], y[3], z[3];
+  __device__ Around(const Geo& g, int i, int j, int k) {
+    const int plane = g.sx * g.ny;
+    x[0] = i == 0 ? g.nx - 1 : i - 1;
+    x[1] = i;
+    x[2] = i == g.nx - 1 ? 0 : i + 1;
+    y[0] = g.sx * (j == 0 ? g.ny - 1 : j - 1);
+    y[1] = g.sx * j;
+    y[2] = g.sx * (j == g.ny - 1 ? 0 : j + 1);
+    z[0] = plane * (k == 0 ? g.nz - 1 : k - 1);
+    z[1] = plane * k;
+    z[2] = plane * (k == g.nz - 1 ? 0 : k + 1);
+  }
+  __device__ int off(int dx, int dy, int dz) const { return x[dx + 1] + y[dy + 1] + z[dz + 1]; }
+};
+
 // ------------------------------------------------------ initial conditions
 // Per-cell equilibrium deviation of SRC/init.F90:97-137 (cte1 = 0):
 // out_q = crho*w_q*(0 + rf*(c.u) + qf*(3*(c.u)^2 - |u|^2)), with each linear
@@ -1108,14 +1147,17 @@ __global__ void k_init_vel(Pops<typename F::S> a, Geo g, int lay, const double* 
                            const double* __restrict__ v, const double* __restrict__ w, double rho, int k0, int nk,
                            typename F::R scale, unsigned int* maxbits) {
   using R = typename F::R; using V = typename F::V; using N = Num<V>;
-  const long long n = (long long)g.nx * g.ny * nk;
   float tmax = 0.f;
-  for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(c % g.nx), j = (int)((c / g.nx) % g.ny), k = k0 + (int)(c / ((long long)g.nx * g.ny));
+  const Units un(g.nx, g.ny, nk);
+  for (unsigned m = blockIdx.x * 8 + (threadIdx.x >> 5); m < un.n; m += gridDim.x * 8) {
+    int i, j, k;
+    un.decode(m, i, j, k);
+    if (i >= g.nx) continue;
+    const long long c = i + (long long)g.nx * (j + (long long)g.ny * k);
     V out[Q];
     eq_init<V>(N::wrap((R)u[c]), N::wrap((R)v[c]), N::wrap((R)w[c]), N::wrap((R)rho), out);
     if (maxbits) tmax = fmaxf(tmax, cell_maxabs<V>(out));
-    else store_cell<F>(a, lay, i + g.sx * (j + g.ny * k), out, scale);
+    else store_cell<F>(a, lay, i + g.sx * (j + g.ny * (k0 + k)), out, scale);
   }
   if (maxbits) atomicMax(maxbits, __float_as_uint(tmax));
 }
@@ -1124,30 +1166,52 @@ __global__ void k_init_vel(Pops<typename F::S> a, Geo g, int lay, const double* 
 // Location of the reference's a_q at cell (i,j,k) + d for a given layout.
 template <int LAY>
 __device__ __forceinline__ int ref_slot(int q) { return LAY == LAY_AAE ? oppq(q) : q; }
-template <int LAY>
-__device__ __forceinline__ int ref_off(const Geo& g, int q, int i, int j, int k, int dx, int dy, int dz) {
-  if (LAY == LAY_AAN) { dx += cxq(q); dy += cyq(q); dz += czq(q); }
-  return wrapi(i + dx, g.nx) + g.sx * (wrapi(j + dy, g.ny) + g.ny * wrapi(k + dz, g.nz));
+// Location of the reference's a_q of the cell (local) and of its pulled a_q,
+// from (x - c_q), for a layout: LAY_AAN keeps a_q of a cell at x + c_q.
+template <int LAY, bool PULL>
+__device__ __forceinline__ int around_off(const Around& n, int q) {
+  constexpr int s = PULL ? (LAY == LAY_AAN ? 0 : -1) : (LAY == LAY_AAN ? 1 : 0);
+  return n.off(s * cxq(q), s * cyq(q), s * czq(q));
 }
 
+// Populations q0 .. q0 + nq - 1 of the reference to nq dense blocks: stored type
+// (out_s) or double deviations (out_d).
 template <class F, int LAY>
-__global__ void k_export(Pops<const typename F::S> a, Geo g, int q, typename F::S* out_s, double* out_d,
-                         typename F::R inv) {
+__global__ void __launch_bounds__(256) k_export(Pops<const typename F::S> a, Geo g, int q0, int nq,
+                                                typename F::S* out_s, double* out_d, typename F::R inv) {
   const long long n = (long long)g.nx * g.ny * g.nz;
-  for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(c % g.nx), j = (int)((c / g.nx) % g.ny), k = (int)(c / ((long long)g.nx * g.ny));
-    const typename F::S s = a.p[ref_slot<LAY>(q)][ref_off<LAY>(g, q, i, j, k, 0, 0, 0)];
-    if (out_s) out_s[c] = s;
-    if (out_d) out_d[c] = (double)F::dec(s, inv);
+  const Units un(g.nx, g.ny, g.nz);
+  for (unsigned u = blockIdx.x * 8 + (threadIdx.x >> 5); u < un.n; u += gridDim.x * 8) {
+    int i, j, k;
+    un.decode(u, i, j, k);
+    if (i >= g.nx) continue;
+    const Around nb(g, i, j, k);
+    const long long c = i + (long long)g.nx * (j + (long long)g.ny * k);
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      if (q < q0 || q >= q0 + nq) continue;
+      const typename F::S s = ldg(a.p[ref_slot<LAY>(q)] + around_off<LAY, false>(nb, q));
+      if (out_s) out_s[(q - q0) * n + c] = s;
+      if (out_d) out_d[(q - q0) * n + c] = (double)F::dec(s, inv);
+    }
   }
 }
 
+// The inverse of k_export's stored form.
 template <class F, int LAY>
-__global__ void k_import(Pops<typename F::S> a, Geo g, int q, const typename F::S* __restrict__ in) {
+__global__ void __launch_bounds__(256) k_import(Pops<typename F::S> a, Geo g, int q0, int nq,
+                                                const typename F::S* __restrict__ in) {
   const long long n = (long long)g.nx * g.ny * g.nz;
-  for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(c % g.nx), j = (int)((c / g.nx) % g.ny), k = (int)(c / ((long long)g.nx * g.ny));
-    a.p[ref_slot<LAY>(q)][ref_off<LAY>(g, q, i, j, k, 0, 0, 0)] = in[c];
+  const Units un(g.nx, g.ny, g.nz);
+  for (unsigned u = blockIdx.x * 8 + (threadIdx.x >> 5); u < un.n; u += gridDim.x * 8) {
+    int i, j, k;
+    un.decode(u, i, j, k);
+    if (i >= g.nx) continue;
+    const Around nb(g, i, j, k);
+    const long long c = i + (long long)g.nx * (j + (long long)g.ny * k);
+#pragma unroll
+    for (int q = 0; q < Q; ++q)
+      if (q >= q0 && q < q0 + nq) a.p[ref_slot<LAY>(q)][around_off<LAY, false>(nb, q)] = in[(q - q0) * n + c];
   }
 }
 
@@ -1197,24 +1261,36 @@ __global__ void k_faith_snapshot(Pops<const S> a, Geo g, S* out) {
   }
 }
 
-template <class F, int LAY, bool FAITH = false>
-__global__ void __launch_bounds__(DIAG_THREADS) k_diag(Pops<const typename F::S> a, Geo g, double svisc,
-                                                       double omega, typename F::R inv, double* partials,
-                                                       typename F::R* vel, Halo<typename F::S> h,
-                                                       const typename F::S* __restrict__ faith, int faith_zero) {
+// Sources of the pulls that leave the box or the slab: the periodic image
+// (PULL_WRAP), the ghost planes of a z-slab (PULL_SLAB), the boundary-plane
+// snapshot of faithful mode (PULL_FAITH).
+enum { PULL_WRAP = 0, PULL_SLAB = 1, PULL_FAITH = 2 };
+constexpr int NDK = 9;  // quantities of k_diag
+
+template <class F, int LAY, int PULL>
+__global__ void __launch_bounds__(DIAG_THREADS, F::id == 0 ? 2 : 3)
+    k_diag(Pops<const typename F::S> a, Geo g, double svisc, double omega, typename F::R inv, double* partials,
+           typename F::R* vel, Halo<typename F::S> h, const typename F::S* __restrict__ faith, int faith_zero) {
   using R = typename F::R; using V = typename F::V; using N = Num<V>;
-  __shared__ KS sh[DIAG_THREADS];
-  KS acc[ND];
+  __shared__ KS sh[DIAG_THREADS / 32][NDK];
+  KS acc[NDK];
 #pragma unroll
-  for (int d = 0; d < ND; ++d) acc[d] = {0.0, 0.0};
+  for (int d = 0; d < NDK; ++d) acc[d] = {0.0, 0.0};
+  int bad = 0;
   const long long n = (long long)g.nx * g.ny * g.nz;
   const V svr = N::wrap((R)svisc);
-  for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(c % g.nx), j = (int)((c / g.nx) % g.ny), k = (int)(c / ((long long)g.nx * g.ny));
+  const double kS = 2.0 * svisc * (9.0 * omega * omega * 0.25);  // 2 nu S:S = kS Ptotal / rho^2
+  const Units un(g.nx, g.ny, g.nz);
+  constexpr unsigned WARPS = DIAG_THREADS / 32;
+  for (unsigned u = blockIdx.x * WARPS + (threadIdx.x >> 5); u < un.n; u += gridDim.x * WARPS) {
+    int i, j, k;
+    un.decode(u, i, j, k);
+    if (i >= g.nx) continue;
+    const Around nb(g, i, j, k);
     V x[Q];
 #pragma unroll
     for (int q = 0; q < Q; ++q)
-      x[q] = N::wrap(F::dec(a.p[ref_slot<LAY>(q)][ref_off<LAY>(g, q, i, j, k, 0, 0, 0)], inv));
+      x[q] = N::wrap(F::dec(ldg(a.p[ref_slot<LAY>(q)] + around_off<LAY, false>(nb, q)), inv));
     V ux, uy, uz;
     const V rho = moments<V>(x, ux, uy, uz);
     const V ke = N::c(0.5) * (ux * ux + uy * uy + uz * uz);
@@ -1223,25 +1299,27 @@ __global__ void __launch_bounds__(DIAG_THREADS) k_diag(Pops<const typename F::S>
     kadd(acc[2], (double)N::raw(uy));
     kadd(acc[3], (double)N::raw(uz));
     kadd(acc[4], (double)N::raw(ke));
-    if (!isfinite(N::raw(rho)) || !isfinite(N::raw(ux)) || !isfinite(N::raw(uy)) || !isfinite(N::raw(uz)))
-      acc[8].s = __dadd_rn(acc[8].s, 1.0);
-    if (vel) { vel[c] = N::raw(ux); vel[n + c] = N::raw(uy); vel[2 * n + c] = N::raw(uz); }
+    if (!isfinite(N::raw(rho)) || !isfinite(N::raw(ux)) || !isfinite(N::raw(uy)) || !isfinite(N::raw(uz))) ++bad;
+    if (vel) {
+      const long long c = i + (long long)g.nx * (j + (long long)g.ny * k);
+      vel[c] = N::raw(ux);
+      vel[n + c] = N::raw(uy);
+      vel[2 * n + c] = N::raw(uz);
+    }
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
-      // a z-slab pulls across its faces from its ghost planes
-      const bool lo = czq(q) > 0 && k == 0, hi = czq(q) < 0 && k == g.nz - 1;
       const int si = i - cxq(q), sj = j - cyq(q), sk = k - czq(q);
-      if (LAY == LAY_TWO && h.in_lo[0] && (lo || hi)) {
-        const int po = wrapi(i - cxq(q), g.nx) + g.sx * wrapi(j - cyq(q), g.ny);
-        x[q] = N::wrap(F::dec(lo ? h.in_lo[zslot(q)][po] : h.in_hi[zslot(q)][po], inv));
-      } else if (FAITH && LAY == LAY_TWO &&
-                 (si < 0 || si >= g.nx || sj < 0 || sj >= g.ny || sk < 0 || sk >= g.nz)) {
+      if (PULL == PULL_SLAB && ((czq(q) > 0 && k == 0) || (czq(q) < 0 && k == g.nz - 1))) {
+        // a z-slab pulls across its faces from its ghost planes
+        const int po = nb.off(-cxq(q), -cyq(q), 0) - nb.z[1];
+        x[q] = N::wrap(F::dec(czq(q) > 0 ? h.in_lo[zslot(q)][po] : h.in_hi[zslot(q)][po], inv));
+      } else if (PULL == PULL_FAITH && (si < 0 || si >= g.nx || sj < 0 || sj >= g.ny || sk < 0 || sk >= g.nz)) {
         // faithful mode: the reference's ghost cell of this pull, filled two
         // steps earlier (or never)
         const long long per = 2 * ((long long)g.ny * g.nz + (long long)g.nx * g.nz + (long long)g.nx * g.ny);
         x[q] = faith_zero ? N::c(0.0) : N::wrap(F::dec(faith[q * per + faith_off(g, si, sj, sk)], inv));
       } else {
-        x[q] = N::wrap(F::dec(a.p[ref_slot<LAY>(q)][ref_off<LAY>(g, q, i, j, k, -cxq(q), -cyq(q), -czq(q))], inv));
+        x[q] = N::wrap(F::dec(ldg(a.p[ref_slot<LAY>(q)] + around_off<LAY, true>(nb, q)), inv));
       }
     }
     V e[Q], vx, vy, vz;
@@ -1250,62 +1328,96 @@ __global__ void __launch_bounds__(DIAG_THREADS) k_diag(Pops<const typename F::S>
     const V P = ptotal<V>(x, e);
     kadd(acc[5], (double)N::raw(N::c(0.5) * vsq));
     kadd(acc[6], (double)N::raw(N::c(2.0) * svr * P));
-    const double r = (double)N::raw(rp);
-    const double eps = __dmul_rn(__dmul_rn(__dmul_rn(2.0, svisc), __ddiv_rn(__dmul_rn(__dmul_rn(9.0, omega), omega),
-                                                                          __dmul_rn(__dmul_rn(4.0, r), r))),
-                                 (double)N::raw(P));
-    kadd(acc[7], eps);
+    const double r = __drcp_rn((double)N::raw(rp));
+    kadd(acc[7], __dmul_rn(__dmul_rn(kS, __dmul_rn(r, r)), (double)N::raw(P)));
   }
+  acc[8].s = (double)bad;
+  const KS r = block_reduce_n<NDK, DIAG_THREADS>(acc, sh);
+  if (threadIdx.x < NDK) {
+    partials[(blockIdx.x * ND + threadIdx.x) * 2 + 0] = r.s;
+    partials[(blockIdx.x * ND + threadIdx.x) * 2 + 1] = r.c;
+  }
+}
+
+// Local velocity j/rho of the cells of planes k0 .. k0 + nk - 1, dense Fortran
+// order (three blocks), in OUT precision: what k_diag also writes, for callers that want nothing else
+// (bgk_get_velocity, bgk_spectrum). 19 loads and 3 stores a cell.
+template <class F, int LAY, class OUT>
+__global__ void __launch_bounds__(256) k_velocity(Pops<const typename F::S> a, Geo g, typename F::R inv, OUT* vel,
+                                                  int k0, int nk) {
+  using V = typename F::V; using N = Num<V>;
+  const long long n = (long long)g.nx * g.ny * nk;
+  const Units un(g.nx, g.ny, nk);
+  for (unsigned u = blockIdx.x * 8 + (threadIdx.x >> 5); u < un.n; u += gridDim.x * 8) {
+    int i, j, k;
+    un.decode(u, i, j, k);
+    if (i >= g.nx) continue;
+    const Around nb(g, i, j, k0 + k);
+    V x[Q];
 #pragma unroll
-  for (int d = 0; d < ND; ++d) {
-    const KS r = block_reduce(acc[d], sh);
-    if (threadIdx.x == 0) {
-      partials[(blockIdx.x * ND + d) * 2 + 0] = r.s;
-      partials[(blockIdx.x * ND + d) * 2 + 1] = r.c;
-    }
+    for (int q = 0; q < Q; ++q)
+      x[q] = N::wrap(F::dec(ldg(a.p[ref_slot<LAY>(q)] + around_off<LAY, false>(nb, q)), inv));
+    V ux, uy, uz;
+    (void)moments<V>(x, ux, uy, uz);
+    const long long c = i + (long long)g.nx * (j + (long long)g.ny * k);
+    vel[c] = (OUT)N::raw(ux);
+    vel[n + c] = (OUT)N::raw(uy);
+    vel[2 * n + c] = (OUT)N::raw(uz);
   }
 }
 
 template <class R>
 __global__ void __launch_bounds__(DIAG_THREADS) k_enstrophy(const R* __restrict__ vel, int nx, int ny, int nz,
                                                             double* partials) {
-  __shared__ KS sh[DIAG_THREADS];
-  KS acc = {0.0, 0.0};
+  __shared__ KS sh[DIAG_THREADS / 32][1];
+  KS acc[1] = {{0.0, 0.0}};
   const long long n = (long long)nx * ny * nz;
-  for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(c % nx), j = (int)((c / nx) % ny), k = (int)(c / ((long long)nx * ny));
+  const Units un(nx, ny, nz);
+  constexpr unsigned WARPS = DIAG_THREADS / 32;
+  for (unsigned u = blockIdx.x * WARPS + (threadIdx.x >> 5); u < un.n; u += gridDim.x * WARPS) {
+    int i, j, k;
+    un.decode(u, i, j, k);
+    if (i >= nx) continue;
     const int ip = i + 1 == nx ? 0 : i + 1, im = i == 0 ? nx - 1 : i - 1;
     const int jp = j + 1 == ny ? 0 : j + 1, jm = j == 0 ? ny - 1 : j - 1;
     const int kp = k + 1 == nz ? 0 : k + 1, km = k == 0 ? nz - 1 : k - 1;
-    auto U = [&](int comp, int a, int b, int d) -> double {
-      return (double)vel[comp * n + a + (long long)nx * (b + (long long)ny * d)];
-    };
+    // rows of the three components at (j, k) and around it
+    const R* const row = vel + (long long)nx * (j + (long long)ny * k);
+    const R* const rjp = vel + (long long)nx * (jp + (long long)ny * k);
+    const R* const rjm = vel + (long long)nx * (jm + (long long)ny * k);
+    const R* const rkp = vel + (long long)nx * (j + (long long)ny * kp);
+    const R* const rkm = vel + (long long)nx * (j + (long long)ny * km);
     using E = Ex<double>;
-    const E h = {0.5};
-    const E dwdy = h * (E{U(2, i, jp, k)} - E{U(2, i, jm, k)});
-    const E dvdz = h * (E{U(1, i, j, kp)} - E{U(1, i, j, km)});
-    const E dudz = h * (E{U(0, i, j, kp)} - E{U(0, i, j, km)});
-    const E dwdx = h * (E{U(2, ip, j, k)} - E{U(2, im, j, k)});
-    const E dvdx = h * (E{U(1, ip, j, k)} - E{U(1, im, j, k)});
-    const E dudy = h * (E{U(0, i, jp, k)} - E{U(0, i, jm, k)});
+    auto D = [&](const R* p, int s, const R* m, int t) -> E { return E{0.5} * (E{(double)__ldg(p + s)} - E{(double)__ldg(m + t)}); };
+    const E dwdy = D(rjp + 2 * n, i, rjm + 2 * n, i), dvdz = D(rkp + n, i, rkm + n, i);
+    const E dudz = D(rkp, i, rkm, i), dwdx = D(row + 2 * n, ip, row + 2 * n, im);
+    const E dvdx = D(row + n, ip, row + n, im), dudy = D(rjp, i, rjm, i);
     const E wx = dwdy - dvdz, wy = dudz - dwdx, wz = dvdx - dudy;
-    kadd(acc, (h * (wx * wx + wy * wy + wz * wz)).v);
+    kadd(acc[0], (E{0.5} * (wx * wx + wy * wy + wz * wz)).v);
   }
-  const KS r = block_reduce(acc, sh);
+  const KS r = block_reduce_n<1, DIAG_THREADS>(acc, sh);
   if (threadIdx.x == 0) {
     partials[(blockIdx.x * ND + 9) * 2 + 0] = r.s;
     partials[(blockIdx.x * ND + 9) * 2 + 1] = r.c;
   }
 }
 
-__global__ void __launch_bounds__(DIAG_THREADS) k_finalize(const double* __restrict__ partials, double* totals) {
-  __shared__ KS sh[DIAG_THREADS];
-  for (int d = 0; d < ND; ++d) {
-    KS acc = {0.0, 0.0};
-    for (int b = threadIdx.x; b < DIAG_BLOCKS; b += blockDim.x)
-      kcomb(acc, KS{partials[(b * ND + d) * 2], partials[(b * ND + d) * 2 + 1]});
-    const KS r = block_reduce(acc, sh);
-    if (threadIdx.x == 0) totals[d] = __dadd_rn(r.s, r.c);
+// One block per quantity (one block for all ten took 16 us). totals may be
+// pinned host memory; err (optional): the device's error flag, copied behind
+// the ND + 1 totals so that the host reads one place.
+__global__ void __launch_bounds__(DIAG_THREADS) k_finalize(const double* __restrict__ partials, double* totals,
+                                                           const int* err) {
+  __shared__ KS sh[DIAG_THREADS / 32][1];
+  const int d = blockIdx.x;
+  KS acc[1] = {{0.0, 0.0}};
+  for (int b = threadIdx.x; b < DIAG_BLOCKS; b += blockDim.x) {
+    const double2 p = __ldg(reinterpret_cast<const double2*>(partials) + b * ND + d);
+    kcomb(acc[0], KS{p.x, p.y});
+  }
+  const KS r = block_reduce_n<1, DIAG_THREADS>(acc, sh);
+  if (threadIdx.x == 0) {
+    totals[d] = __dadd_rn(r.s, r.c);
+    if (d == 0 && err) totals[ND + 1] = (double)*err;
   }
 }
 
@@ -1313,9 +1425,11 @@ template <class F, int LAY>
 __global__ void k_last_zj(Pops<const typename F::S> a, Geo g, typename F::R inv, double* out) {
   using V = typename F::V; using N = Num<V>;
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
+  const Around nb(g, g.nx - 1, g.ny - 1, g.nz - 1);
   V x[Q];
+#pragma unroll
   for (int q = 0; q < Q; ++q)
-    x[q] = N::wrap(F::dec(a.p[ref_slot<LAY>(q)][ref_off<LAY>(g, q, g.nx - 1, g.ny - 1, g.nz - 1, 0, 0, 0)], inv));
+    x[q] = N::wrap(F::dec(a.p[ref_slot<LAY>(q)][around_off<LAY, false>(nb, q)], inv));
   V ux, uy, uz;
   (void)moments<V>(x, ux, uy, uz);
   *out = (double)N::raw(uz);
@@ -1337,9 +1451,10 @@ __global__ void k_vtk(Pops<const typename F::S> a, Geo g, int kind, int index, f
     else if (kind == 2) { i = (int)(c % g.nx); k = (int)(c / g.nx); j = index; }
     else if (kind == 3) { j = (int)(c % g.ny); k = (int)(c / g.ny); i = index; }
     else { i = (int)(c % g.nx); j = (int)((c / g.nx) % g.ny); k = (int)(c / ((long long)g.nx * g.ny)); }
+    const Around nb(g, i, j, k);
     V x[Q];
 #pragma unroll
-    for (int q = 0; q < Q; ++q) x[q] = N::wrap(F::dec(a.p[ref_slot<LAY>(q)][ref_off<LAY>(g, q, i, j, k, 0, 0, 0)], inv));
+    for (int q = 0; q < Q; ++q) x[q] = N::wrap(F::dec(a.p[ref_slot<LAY>(q)][around_off<LAY, false>(nb, q)], inv));
     const V u = x[0] + x[1] + x[2] + x[3] + x[4] - x[9] - x[10] - x[11] - x[12] - x[13];
     const V w = x[2] + x[6] + x[7] + x[8] + x[11] - x[0] - x[9] - x[15] - x[16] - x[17];
     const V v = x[3] + x[5] + x[6] + x[12] + x[17] - x[1] - x[8] - x[10] - x[14] - x[15];
@@ -1353,14 +1468,73 @@ __global__ void k_vtk(Pops<const typename F::S> a, Geo g, int kind, int index, f
 }
 
 // --------------------------------------------------------------- spectrum
+// Shell of a wavevector: floor(|k| + 1/2), in integers (b^2 - b < |k|^2 <= b^2 + b).
+__device__ __forceinline__ int shell_of(int k2) {
+  int b = (int)(__fsqrt_rn((float)k2) + 0.5f);
+  if (k2 > b * b + b) ++b;
+  else if (b > 0 && k2 <= b * b - b) --b;
+  return b;
+}
+
+constexpr int SPEC_WARPS = 8;
+constexpr int SPEC_MAX_SIDE = 16384;  // |k|^2 and b^2 + b stay below 2^31
+
+// One transformed component into the shells. A warp takes 32 consecutive modes
+// of a row, whose shells never decrease from lane to lane (kx >= 0): a segmented
+// sum over the lanes leaves one value per shell, added without atomics to the
+// warp's own table in shared memory; the block adds its tables to the result
+// at the end. (A global atomic per mode took 1060 us per component at 256^3
+// FP64, against 21 us for reading it at the copy rate.)
 template <class C>
-__global__ void k_spec_bins(const C* __restrict__ f, int nx, int ny, int nz, int nbins, double* bins, double norm) {
+__global__ void __launch_bounds__(32 * SPEC_WARPS) k_spec_bins(const C* __restrict__ f, int nx, int ny, int nz,
+                                                               int nb, double* bins, double norm) {
+  extern __shared__ double tab[];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int b = threadIdx.x; b < SPEC_WARPS * nb; b += blockDim.x) tab[b] = 0.0;
+  __syncthreads();
+  double* const own = tab + w * nb;
+  const int nxh = nx / 2 + 1;
+  const Units un(nxh, ny, nz);
+  for (unsigned u = blockIdx.x * SPEC_WARPS + w; u < un.n; u += gridDim.x * SPEC_WARPS) {
+    int ix, iy, iz;
+    un.decode(u, ix, iy, iz);
+    const int ky = iy <= ny / 2 ? iy : iy - ny, kz = iz <= nz / 2 ? iz : iz - nz;
+    double v = 0.0;
+    int b = nb;
+    if (ix < nxh) {
+      const C c = f[ix + (long long)nxh * (iy + (long long)ny * iz)];
+      // modes 0 < kx < nx/2 stand for their conjugate partner as well
+      const double wt = (ix == 0 || (nx % 2 == 0 && ix == nx / 2)) ? 1.0 : 2.0;
+      const double re = (double)c.x, im = (double)c.y;
+      v = wt * 0.5 * (re * re + im * im) * norm;
+      b = min(nb, shell_of(ix * ix + ky * ky + kz * kz));
+    }
+#pragma unroll
+    for (int s = 1; s < 32; s <<= 1) {
+      const double o = __shfl_up_sync(0xffffffffu, v, s);
+      const int ob = __shfl_up_sync(0xffffffffu, b, s);
+      if (lane >= s && ob == b) v += o;
+    }
+    const int next = __shfl_down_sync(0xffffffffu, b, 1);
+    if (b < nb && (lane == 31 || next != b)) own[b] += v;
+    __syncwarp();
+  }
+  __syncthreads();
+  for (int b = threadIdx.x; b < nb; b += blockDim.x) {
+    double v = 0.0;
+    for (int m = 0; m < SPEC_WARPS; ++m) v += tab[m * nb + b];
+    if (v != 0.0) atomicAdd(bins + b, v);
+  }
+}
+
+// The same for boxes whose shells do not fit the tables: one atomic per mode.
+template <class C>
+__global__ void k_spec_bins_any(const C* __restrict__ f, int nx, int ny, int nz, int nbins, double* bins, double norm) {
   const int nxh = nx / 2 + 1;
   const long long n = (long long)nxh * ny * nz;
   for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x) {
     const int ix = (int)(c % nxh), iy = (int)((c / nxh) % ny), iz = (int)(c / ((long long)nxh * ny));
     const int ky = iy <= ny / 2 ? iy : iy - ny, kz = iz <= nz / 2 ? iz : iz - nz;
-    // modes 0 < kx < nx/2 stand for their conjugate partner as well
     const double w = (ix == 0 || (nx % 2 == 0 && ix == nx / 2)) ? 1.0 : 2.0;
     const double kk = sqrt((double)ix * ix + (double)ky * ky + (double)kz * kz);
     const int b = (int)floor(kk + 0.5);
@@ -1371,15 +1545,26 @@ __global__ void k_spec_bins(const C* __restrict__ f, int nx, int ny, int nz, int
   }
 }
 
+template <class C>
+static cudaError_t spec_impl(const void* fft_out, int nx, int ny, int nz, int nbins, double* bins, double norm,
+                             cudaStream_t st) {
+  const double kmax = std::sqrt(0.25 * ((double)nx * nx + (double)ny * ny + (double)nz * nz));
+  const int nb = (int)std::min((double)nbins, std::floor(kmax + 0.5) + 1.0);  // shells above hold nothing
+  const size_t bytes = (size_t)SPEC_WARPS * nb * sizeof(double);
+  if (nx <= SPEC_MAX_SIDE && ny <= SPEC_MAX_SIDE && nz <= SPEC_MAX_SIDE && bytes <= 48 * 1024) {
+    const int grid = grid_1d(Units(nx / 2 + 1, ny, nz).n, SPEC_WARPS, 148 * 4);
+    k_spec_bins<C><<<grid, 32 * SPEC_WARPS, bytes, st>>>((const C*)fft_out, nx, ny, nz, nb, bins, norm);
+  } else {
+    const long long n = (long long)(nx / 2 + 1) * ny * nz;
+    k_spec_bins_any<C><<<grid_1d(n, 256, 148 * 16), 256, 0, st>>>((const C*)fft_out, nx, ny, nz, nbins, bins, norm);
+  }
+  return cudaGetLastError();
+}
+
 cudaError_t launch_spectrum_bins(const void* fft_out, int form, int nx, int ny, int nz, int nbins, double* bins,
                                  double norm, cudaStream_t st) {
-  const long long n = (long long)(nx / 2 + 1) * ny * nz;
-  const int grid = grid_1d(n, 256, 148 * 16);
-  if (form == FORM_F64)
-    k_spec_bins<double2><<<grid, 256, 0, st>>>((const double2*)fft_out, nx, ny, nz, nbins, bins, norm);
-  else
-    k_spec_bins<float2><<<grid, 256, 0, st>>>((const float2*)fft_out, nx, ny, nz, nbins, bins, norm);
-  return cudaGetLastError();
+  return form == FORM_F64 ? spec_impl<double2>(fft_out, nx, ny, nz, nbins, bins, norm, st)
+                          : spec_impl<float2>(fft_out, nx, ny, nz, nbins, bins, norm, st);
 }
 
 // ---------------------------------------------------------------- shift3
@@ -1633,8 +1818,7 @@ template <class F>
 static cudaError_t vel_impl(const Lattice& a, int lay, const double* u, const double* v, const double* w, double rho,
                             int k0, int nk, double scale, unsigned int* mx, cudaStream_t st) {
   using S = typename F::S; using R = typename F::R;
-  const long long n = (long long)a.g.nx * a.g.ny * nk;
-  k_init_vel<F><<<grid_1d(n, 256, 148 * 32), 256, 0, st>>>(pops_of<S>(a), a.g, lay, u, v, w, rho, k0, nk, (R)scale,
+  k_init_vel<F><<<grid_1d(Units(a.g.nx, a.g.ny, nk).n, 8, 148 * 32), 256, 0, st>>>(pops_of<S>(a), a.g, lay, u, v, w, rho, k0, nk, (R)scale,
                                                            mx);
   return cudaGetLastError();
 }
@@ -1649,47 +1833,48 @@ cudaError_t launch_init_velocity(const Lattice& a, int lay, const double* u, con
   return cudaErrorInvalidValue;
 }
 
+static int unit_grid(const Geo& g) { return grid_1d(Units(g.nx, g.ny, g.nz).n, 8, 148 * 32); }
+
 template <class F, int LAY>
-static void export_lay(const Lattice& a, int q, void* ds, double* dd, double scale, cudaStream_t st) {
+static void export_lay(const Lattice& a, int q0, int nq, void* ds, double* dd, double scale, cudaStream_t st) {
   using S = typename F::S; using R = typename F::R;
-  const long long n = (long long)a.g.nx * a.g.ny * a.g.nz;
-  k_export<F, LAY><<<grid_1d(n, 256, 148 * 32), 256, 0, st>>>(pops_of<const S>(a), a.g, q, (S*)ds, dd,
-                                                               (R)(1.0 / scale));
+  k_export<F, LAY><<<unit_grid(a.g), 256, 0, st>>>(pops_of<const S>(a), a.g, q0, nq, (S*)ds, dd, (R)(1.0 / scale));
 }
 template <class F>
-static cudaError_t export_impl(const Lattice& a, int lay, int q, void* ds, double* dd, double scale, cudaStream_t st) {
-  if (lay == LAY_TWO) export_lay<F, LAY_TWO>(a, q, ds, dd, scale, st);
-  else if (lay == LAY_AAE) export_lay<F, LAY_AAE>(a, q, ds, dd, scale, st);
-  else export_lay<F, LAY_AAN>(a, q, ds, dd, scale, st);
+static cudaError_t export_impl(const Lattice& a, int lay, int q0, int nq, void* ds, double* dd, double scale,
+                               cudaStream_t st) {
+  if (lay == LAY_TWO) export_lay<F, LAY_TWO>(a, q0, nq, ds, dd, scale, st);
+  else if (lay == LAY_AAE) export_lay<F, LAY_AAE>(a, q0, nq, ds, dd, scale, st);
+  else export_lay<F, LAY_AAN>(a, q0, nq, ds, dd, scale, st);
   return cudaGetLastError();
 }
-cudaError_t launch_export(const Lattice& a, int lay, int q, void* ds, double* dd, double scale, cudaStream_t st) {
+cudaError_t launch_export(const Lattice& a, int lay, int q0, int nq, void* ds, double* dd, double scale,
+                          cudaStream_t st) {
   switch (a.form) {
-    case FORM_F64: return export_impl<F64>(a, lay, q, ds, dd, scale, st);
-    case FORM_F32: return export_impl<F32>(a, lay, q, ds, dd, scale, st);
-    case FORM_F16: return export_impl<F16>(a, lay, q, ds, dd, scale, st);
+    case FORM_F64: return export_impl<F64>(a, lay, q0, nq, ds, dd, scale, st);
+    case FORM_F32: return export_impl<F32>(a, lay, q0, nq, ds, dd, scale, st);
+    case FORM_F16: return export_impl<F16>(a, lay, q0, nq, ds, dd, scale, st);
   }
   return cudaErrorInvalidValue;
 }
 
 template <class F, int LAY>
-static void import_lay(const Lattice& a, int q, const void* ds, cudaStream_t st) {
+static void import_lay(const Lattice& a, int q0, int nq, const void* ds, cudaStream_t st) {
   using S = typename F::S;
-  const long long n = (long long)a.g.nx * a.g.ny * a.g.nz;
-  k_import<F, LAY><<<grid_1d(n, 256, 148 * 32), 256, 0, st>>>(pops_of<S>(a), a.g, q, (const S*)ds);
+  k_import<F, LAY><<<unit_grid(a.g), 256, 0, st>>>(pops_of<S>(a), a.g, q0, nq, (const S*)ds);
 }
 template <class F>
-static cudaError_t import_impl(const Lattice& a, int lay, int q, const void* ds, cudaStream_t st) {
-  if (lay == LAY_TWO) import_lay<F, LAY_TWO>(a, q, ds, st);
-  else if (lay == LAY_AAE) import_lay<F, LAY_AAE>(a, q, ds, st);
-  else import_lay<F, LAY_AAN>(a, q, ds, st);
+static cudaError_t import_impl(const Lattice& a, int lay, int q0, int nq, const void* ds, cudaStream_t st) {
+  if (lay == LAY_TWO) import_lay<F, LAY_TWO>(a, q0, nq, ds, st);
+  else if (lay == LAY_AAE) import_lay<F, LAY_AAE>(a, q0, nq, ds, st);
+  else import_lay<F, LAY_AAN>(a, q0, nq, ds, st);
   return cudaGetLastError();
 }
-cudaError_t launch_import(const Lattice& a, int lay, int q, const void* ds, cudaStream_t st) {
+cudaError_t launch_import(const Lattice& a, int lay, int q0, int nq, const void* ds, cudaStream_t st) {
   switch (a.form) {
-    case FORM_F64: return import_impl<F64>(a, lay, q, ds, st);
-    case FORM_F32: return import_impl<F32>(a, lay, q, ds, st);
-    case FORM_F16: return import_impl<F16>(a, lay, q, ds, st);
+    case FORM_F64: return import_impl<F64>(a, lay, q0, nq, ds, st);
+    case FORM_F32: return import_impl<F32>(a, lay, q0, nq, ds, st);
+    case FORM_F16: return import_impl<F16>(a, lay, q0, nq, ds, st);
   }
   return cudaErrorInvalidValue;
 }
@@ -1706,25 +1891,49 @@ template <class S> static Halo<S> halo_of(const SlabLinks* l) {
   return h;
 }
 
-template <class F, int LAY>
-static void diag_lay(const Lattice& a, double svisc, double omega, double scale, double* partials, void* vel,
-                     const SlabLinks* halo, const void* faith, bool fzero, cudaStream_t st) {
+template <class F, int LAY, int PULL>
+static void diag_pull(const Lattice& a, double svisc, double omega, double scale, double* partials, void* vel,
+                      const SlabLinks* halo, const void* faith, bool fzero, cudaStream_t st) {
   using S = typename F::S; using R = typename F::R;
-  if (faith || fzero)
-    k_diag<F, LAY, true><<<DIAG_BLOCKS, DIAG_THREADS, 0, st>>>(pops_of<const S>(a), a.g, svisc, omega,
-                                                             (R)(1.0 / scale), partials, (R*)vel, halo_of<S>(halo),
-                                                             (const S*)faith, fzero ? 1 : 0);
-  else
-    k_diag<F, LAY><<<DIAG_BLOCKS, DIAG_THREADS, 0, st>>>(pops_of<const S>(a), a.g, svisc, omega, (R)(1.0 / scale),
-                                                         partials, (R*)vel, halo_of<S>(halo), nullptr, 0);
+  k_diag<F, LAY, PULL><<<DIAG_BLOCKS, DIAG_THREADS, 0, st>>>(pops_of<const S>(a), a.g, svisc, omega, (R)(1.0 / scale),
+                                                            partials, (R*)vel, halo_of<S>(halo), (const S*)faith,
+                                                            fzero ? 1 : 0);
 }
 template <class F>
 static cudaError_t diag_impl(const Lattice& a, int lay, double svisc, double omega, double scale, double* partials,
                              void* vel, const SlabLinks* halo, const void* faith, bool fzero, cudaStream_t st) {
-  if (lay == LAY_TWO) diag_lay<F, LAY_TWO>(a, svisc, omega, scale, partials, vel, halo, faith, fzero, st);
-  else if (lay == LAY_AAE) diag_lay<F, LAY_AAE>(a, svisc, omega, scale, partials, vel, halo, nullptr, false, st);
-  else diag_lay<F, LAY_AAN>(a, svisc, omega, scale, partials, vel, halo, nullptr, false, st);
+  if (lay == LAY_AAE) diag_pull<F, LAY_AAE, PULL_WRAP>(a, svisc, omega, scale, partials, vel, nullptr, nullptr, false, st);
+  else if (lay == LAY_AAN) diag_pull<F, LAY_AAN, PULL_WRAP>(a, svisc, omega, scale, partials, vel, nullptr, nullptr, false, st);
+  else if (halo) diag_pull<F, LAY_TWO, PULL_SLAB>(a, svisc, omega, scale, partials, vel, halo, nullptr, false, st);
+  else if (faith || fzero) diag_pull<F, LAY_TWO, PULL_FAITH>(a, svisc, omega, scale, partials, vel, nullptr, faith, fzero, st);
+  else diag_pull<F, LAY_TWO, PULL_WRAP>(a, svisc, omega, scale, partials, vel, nullptr, nullptr, false, st);
   return cudaGetLastError();
+}
+
+template <class F, class OUT>
+static cudaError_t velocity_impl(const Lattice& a, int lay, double scale, void* vel, int k0, int nk,
+                                 cudaStream_t st) {
+  using S = typename F::S; using R = typename F::R;
+  const Units un(a.g.nx, a.g.ny, nk);
+  const int grid = grid_1d(un.n, 8, 148 * 32);
+  const R inv = (R)(1.0 / scale);
+  if (lay == LAY_TWO) k_velocity<F, LAY_TWO, OUT><<<grid, 256, 0, st>>>(pops_of<const S>(a), a.g, inv, (OUT*)vel, k0, nk);
+  else if (lay == LAY_AAE) k_velocity<F, LAY_AAE, OUT><<<grid, 256, 0, st>>>(pops_of<const S>(a), a.g, inv, (OUT*)vel, k0, nk);
+  else k_velocity<F, LAY_AAN, OUT><<<grid, 256, 0, st>>>(pops_of<const S>(a), a.g, inv, (OUT*)vel, k0, nk);
+  return cudaGetLastError();
+}
+cudaError_t launch_velocity(const Lattice& a, int lay, double scale, void* vel, bool as_double, int k0, int nk,
+                            cudaStream_t st) {
+  switch (a.form) {
+    case FORM_F64: return velocity_impl<F64, double>(a, lay, scale, vel, k0, nk, st);
+    case FORM_F32:
+      return as_double ? velocity_impl<F32, double>(a, lay, scale, vel, k0, nk, st)
+                       : velocity_impl<F32, float>(a, lay, scale, vel, k0, nk, st);
+    case FORM_F16:
+      return as_double ? velocity_impl<F16, double>(a, lay, scale, vel, k0, nk, st)
+                       : velocity_impl<F16, float>(a, lay, scale, vel, k0, nk, st);
+  }
+  return cudaErrorInvalidValue;
 }
 
 long long faith_planes_elems(const Geo& g) {
@@ -1829,8 +2038,8 @@ cudaError_t launch_enstrophy(const Lattice& a, const void* vel, double* partials
   return cudaGetLastError();
 }
 
-cudaError_t launch_finalize(const double* partials, double* totals, cudaStream_t st) {
-  k_finalize<<<1, DIAG_THREADS, 0, st>>>(partials, totals);
+cudaError_t launch_finalize(const double* partials, double* totals, cudaStream_t st, const int* err) {
+  k_finalize<<<ND, DIAG_THREADS, 0, st>>>(partials, totals, err);
   return cudaGetLastError();
 }
 

@@ -98,10 +98,10 @@ cudaError_t launch_init_tgv(const Lattice& a, int lay, double u0, int faithful, 
 cudaError_t launch_init_velocity(const Lattice& a, int lay, const double* u, const double* v, const double* w,
                                  double rho, int k0, int nk, double scale, unsigned int* mx, cudaStream_t st);
 
-// Population q in reference semantics, dense Fortran order.
-cudaError_t launch_export(const Lattice& a, int lay, int q, void* dense_stored, double* dense_dev, double scale,
-                          cudaStream_t st);
-cudaError_t launch_import(const Lattice& a, int lay, int q, const void* dense_stored, cudaStream_t st);
+// Populations q0 .. q0 + nq - 1 in reference semantics, dense Fortran order.
+cudaError_t launch_export(const Lattice& a, int lay, int q0, int nq, void* dense_stored, double* dense_dev,
+                          double scale, cudaStream_t st);
+cudaError_t launch_import(const Lattice& a, int lay, int q0, int nq, const void* dense_stored, cudaStream_t st);
 
 // Faithful-mode ghosts: the six boundary planes (x = 0, nx-1; y = 0, ny-1;
 // z = 0, nz-1) of every population of a two-lattice state, stored type,
@@ -128,8 +128,13 @@ cudaError_t launch_slab(const Lattice& src, const Lattice& dst, const SlabLinks&
                         double les_cs, cudaStream_t st, cudaStream_t st_interior);
 cudaError_t launch_halo_prime(const Lattice& a, const SlabLinks& links, cudaStream_t st);
 cudaError_t launch_enstrophy(const Lattice& a, const void* vel, double* partials, cudaStream_t st);
-// Sums DIAG_BLOCKS partials into ND totals (fixed order, compensated).
-cudaError_t launch_finalize(const double* partials, double* totals, cudaStream_t st);
+// Local velocity of the cells of planes k0 .. k0 + nk - 1 (three dense blocks,
+// as double or in the form's arithmetic type), nothing else.
+cudaError_t launch_velocity(const Lattice& a, int lay, double scale, void* vel, bool as_double, int k0, int nk,
+                            cudaStream_t st);
+// Sums DIAG_BLOCKS partials into ND totals (fixed order, compensated); with
+// err, also the error flag as totals[ND + 1]. totals: device or pinned host.
+cudaError_t launch_finalize(const double* partials, double* totals, cudaStream_t st, const int* err = nullptr);
 // Faithful-mode helper: zj of the last cell (i=l, j=m, k=n) into *out.
 cudaError_t launch_last_zj(const Lattice& a, int lay, double scale, double* out, cudaStream_t st);
 

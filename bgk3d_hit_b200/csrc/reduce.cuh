@@ -1,16 +1,19 @@
 // Deterministic compensated FP64 reductions shared by the diagnostics and
-// the adjoint: Neumaier pairs per thread, fixed-order block trees.
+// the adjoint: compensated (sum, error) pairs per thread, fixed-order block
+// trees.
 #pragma once
 #include <cuda_runtime.h>
 
 namespace bgk {
 
 struct KS { double s, c; };
-// Neumaier step; explicit _rn operations keep it free of FMA contraction.
+// Compensated step: the exact rounding error of a.s + v (Knuth's TwoSum, no
+// comparison of the magnitudes) goes into a.c. Explicit _rn operations keep it
+// free of FMA contraction.
 __device__ __forceinline__ void kadd(KS& a, double v) {
   const double t = __dadd_rn(a.s, v);
-  if (fabs(a.s) >= fabs(v)) a.c = __dadd_rn(a.c, __dadd_rn(__dsub_rn(a.s, t), v));
-  else a.c = __dadd_rn(a.c, __dadd_rn(__dsub_rn(v, t), a.s));
+  const double z = __dsub_rn(t, a.s);
+  a.c = __dadd_rn(a.c, __dadd_rn(__dsub_rn(a.s, __dsub_rn(t, z)), __dsub_rn(v, z)));
   a.s = t;
 }
 __device__ __forceinline__ void kcomb(KS& a, const KS& b) {
@@ -29,6 +32,32 @@ __device__ __forceinline__ KS block_reduce(KS v, KS* sh) {
   }
   KS r = sh[0];
   __syncthreads();
+  return r;
+}
+
+// The same for N quantities at once: shuffles inside the warps, then one thread
+// per quantity over the warps' pairs, so a block pays two barriers instead of
+// a shared-memory tree per quantity (nine of them were 9 us of the 22 us that
+// the diagnostics of a 32^3 box took). Thread d < N returns quantity d.
+template <int N, int THREADS>
+__device__ __forceinline__ KS block_reduce_n(KS (&v)[N], KS (&sh)[THREADS / 32][N]) {
+  static_assert(THREADS % 32 == 0 && N <= THREADS, "whole warps");
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+  for (int d = 0; d < N; ++d) {
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) {
+      const KS o = {__shfl_down_sync(0xffffffffu, v[d].s, s), __shfl_down_sync(0xffffffffu, v[d].c, s)};
+      kcomb(v[d], o);
+    }
+    if (lane == 0) sh[w][d] = v[d];
+  }
+  __syncthreads();
+  KS r = {0.0, 0.0};
+  if (threadIdx.x < N) {
+    r = sh[0][threadIdx.x];
+    for (int m = 1; m < THREADS / 32; ++m) kcomb(r, sh[m][threadIdx.x]);
+  }
   return r;
 }
 
