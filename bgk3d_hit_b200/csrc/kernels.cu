@@ -8,11 +8,11 @@
 //   k_two_f32v, k_aa_f32v / k_two_f16v, k_aa_f16v
 //                the same updates with two FP32 / four FP16 cells of a row per
 //                thread (8-byte accesses, x-crossing values by warp shuffle);
-//                the defaults of those forms where a box fits them
+//                the defaults of those forms from VEC_MIN_* cells
 //   k_aa_f16w, k_aa_f32w
 //                the AA odd step with eight FP16 (BGK) / four FP32 (BGK and
 //                Smagorinsky) cells per thread, 16-byte accesses: its default
-//                where a box fits it
+//                where rows are whole chunks
 //   k_slab       two-lattice step of one z-slab with the face exchange fused in
 //   k_init_*     equilibrium initial conditions (SRC/init.F90:83-141)
 //   k_diag       diagno + dissipation + strain-rate sums (SRC/diagno.F90:73-121,
@@ -74,8 +74,11 @@ __global__ void __launch_bounds__(256) k_two(Pops<const typename F::S> src, Pops
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z;
-  if (i >= g.nx || j >= g.ny) return;
-  const int im = i == 0 ? g.nx - 1 : i - 1, ip = i == g.nx - 1 ? 0 : i + 1;
+  // a row's threads run on to the end of its last 32-byte sector (padding, which
+  // reaches no cell): a partly written sector costs memory a read
+  constexpr int P = 32 / sizeof(S);
+  if (i >= (g.nx + P - 1) / P * P || j >= g.ny) return;
+  const int im = i == 0 ? g.nx - 1 : i - 1, ip = i >= g.nx - 1 ? 0 : i + 1;
   const int jm = j == 0 ? g.ny - 1 : j - 1, jp = j == g.ny - 1 ? 0 : j + 1;
   const int km = k == 0 ? g.nz - 1 : k - 1, kp = k == g.nz - 1 ? 0 : k + 1;
   S v[Q];
@@ -97,7 +100,7 @@ __global__ void __launch_bounds__(256) k_two(Pops<const typename F::S> src, Pops
 }
 
 // FP16 two-lattice step with 4 cells per thread and 8-byte accesses. A row of
-// nx cells is handled by tpr = nx/4 consecutive threads (tpr a power of two).
+// nx cells is handled by tpr consecutive threads (VecPlace).
 // x-shifted pulls take the element that crosses a thread boundary from the
 // neighbouring lane (warp shuffle); across warp boundaries (tpr > 32) lanes 0
 // and 31 load it. Each cell's arithmetic is F16::cell's (moments16, pair16,
@@ -109,20 +112,16 @@ __global__ void __launch_bounds__(256) k_two(Pops<const typename F::S> src, Pops
 // variant 78.5 against 67.9 with 108 spilled bytes); earlier forms of the
 // kernel measured 76.6 with 256-thread blocks, 64.5 for all four cells at once
 // at 2 blocks per SM and 58.4 at 64 registers (heavy spills).
-template <bool LES>
+template <bool LES, bool FLAT>
 __global__ void __launch_bounds__(128, 5) k_two_f16v(Pops<const __half> src, Pops<__half> dst, Geo g, StepK K,
-                                                  int log_tpr, int k0) {
-  const int tpr = 1 << log_tpr;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = t >> log_tpr, pos = t & (tpr - 1);
+                                                  int rows, int k0) {
+  const VecPlace<4, FLAT> at(g, rows);
   const int k = blockIdx.y + k0;  // planes k0 .. k0 + gridDim.y - 1
-  if (j >= g.ny) return;  // whole warps: ny*tpr is a multiple of 32
-  const XLanes xl(tpr, pos, threadIdx.x & 31);
-  const int i0 = pos * 4;
+  if (!at.valid) return;  // whole warps unless FLAT; no lane needs a value of theirs
+  const XLanes xl(at, threadIdx.x & 31);
+  const int j = at.j, i0 = at.i0;
   const int jm = j == 0 ? g.ny - 1 : j - 1, jp = j == g.ny - 1 ? 0 : j + 1;
   const int km = k == 0 ? g.nz - 1 : k - 1, kp = k == g.nz - 1 ? 0 : k + 1;
-  const int i_prev = pos == 0 ? g.nx - 1 : i0 - 1;
-  const int i_next = pos == tpr - 1 ? 0 : i0 + 4;
   uint2 Y[Q];  // four cells' stored values per population, cell m in half m
   unsigned short E[Q];
 #pragma unroll
@@ -132,9 +131,10 @@ __global__ void __launch_bounds__(128, 5) k_two_f16v(Pops<const __half> src, Pop
     const __half* p = (q == Q - 1 ? (const __half*)dst.p[Q - 1] : src.p[q]) + g.sx * (jj + g.ny * kk);
     Y[q] = (q == Q - 1) ? *reinterpret_cast<const uint2*>(p + i0) : __ldg(reinterpret_cast<const uint2*>(p + i0));
     E[q] = 0;
-    if (cxq(q) > 0 && xl.edge_prev) E[q] = ldg_u16(p + i_prev);
-    if (cxq(q) < 0 && xl.edge_next) E[q] = ldg_u16(p + i_next);
+    if (cxq(q) > 0 && xl.edge_prev) E[q] = ldg_u16(p + at.i_prev);
+    if (cxq(q) < 0 && xl.edge_next) E[q] = ldg_u16(p + at.i_next);
   }
+  if (at.last()) wrap_last(Y, E, at.cells);
   shift_rows(Y, E, xl);
   collide4_f16<LES>(Y, K);
   const int o = i0 + g.sx * (j + g.ny * k);
@@ -143,24 +143,20 @@ __global__ void __launch_bounds__(128, 5) k_two_f16v(Pops<const __half> src, Pop
 }
 
 // FP32 two-lattice step with 2 cells per thread and 8-byte accesses (tpr =
-// nx/2 threads per row): k_two_f16v's row split and x-crossing shuffles on
+// chunks of a row): k_two_f16v's row split and x-crossing shuffles on
 // chunks of two floats, F32::cell's arithmetic on each cell, so the results
 // are those of k_two<F32>. 72 registers (80 for the Smagorinsky step), no
 // spills.
-template <bool LES>
+template <bool LES, bool FLAT>
 __global__ void __launch_bounds__(128, 5) k_two_f32v(Pops<const float> src, Pops<float> dst, Geo g, StepK K,
-                                                  int log_tpr, int k0) {
-  const int tpr = 1 << log_tpr;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = t >> log_tpr, pos = t & (tpr - 1);
+                                                  int rows, int k0) {
+  const VecPlace<2, FLAT> at(g, rows);
   const int k = blockIdx.y + k0;  // planes k0 .. k0 + gridDim.y - 1
-  if (j >= g.ny) return;  // whole warps: ny*tpr is a multiple of 32
-  const XLanes xl(tpr, pos, threadIdx.x & 31);
-  const int i0 = pos * 2;
+  if (!at.valid) return;  // whole warps unless FLAT; no lane needs a value of theirs
+  const XLanes xl(at, threadIdx.x & 31);
+  const int j = at.j, i0 = at.i0;
   const int jm = j == 0 ? g.ny - 1 : j - 1, jp = j == g.ny - 1 ? 0 : j + 1;
   const int km = k == 0 ? g.nz - 1 : k - 1, kp = k == g.nz - 1 ? 0 : k + 1;
-  const int i_prev = pos == 0 ? g.nx - 1 : i0 - 1;
-  const int i_next = pos == tpr - 1 ? 0 : i0 + 2;
   float2 Y[Q];  // two cells' values per population, cell m in component m
   float E[Q];
 #pragma unroll
@@ -172,9 +168,10 @@ __global__ void __launch_bounds__(128, 5) k_two_f32v(Pops<const float> src, Pops
     const float* p = src.p[q] + g.sx * (jj + g.ny * kk);
     Y[q] = (q == Q - 1) ? *reinterpret_cast<const float2*>(p + i0) : __ldg(reinterpret_cast<const float2*>(p + i0));
     E[q] = 0.f;
-    if (cxq(q) > 0 && xl.edge_prev) E[q] = __ldg(p + i_prev);
-    if (cxq(q) < 0 && xl.edge_next) E[q] = __ldg(p + i_next);
+    if (cxq(q) > 0 && xl.edge_prev) E[q] = __ldg(p + at.i_prev);
+    if (cxq(q) < 0 && xl.edge_next) E[q] = __ldg(p + at.i_next);
   }
+  if (at.last()) wrap_last(Y, E, at.cells);
   shift_rows_f32(Y, E, xl);
 #pragma unroll
   for (int m = 0; m < 2; ++m) {
@@ -349,59 +346,64 @@ __global__ void __launch_bounds__(256, 5) k_aa_f16_odd(Pops<__half> a, Geo g, St
 // skipping its store of the crossing element; at block boundaries the edge
 // lanes store their part of the chunk and their crossing value with 4- and
 // 2-byte stores.
-__device__ __forceinline__ void shift_out(uint2 Y, int cx, __half* p, int i0, int i_prev, int i_next,
-                                              const XLanes& xl, bool prev_in, bool next_in, unsigned from_prev,
-                                              unsigned from_next) {
+template <bool FLAT>
+__device__ __forceinline__ void shift_out(uint2 Y, int cx, __half* p, const VecPlace<4, FLAT>& at, const XLanes& xl,
+                                          const EdgeWarps& ew, unsigned from_prev, unsigned from_next) {
+  const int i0 = at.i0;
   unsigned short* u = reinterpret_cast<unsigned short*>(p);
   if (cx == 0) {
     *reinterpret_cast<uint2*>(p + i0) = Y;
   } else if (cx > 0) {  // cell i0+m -> element i0+m+1
     unsigned prev = __shfl_sync(0xffffffffu, Y.y >> 16, xl.src_prev);  // cell i0-1 of the lane before
-    if (xl.edge_prev && prev_in) prev = from_prev;
+    if (xl.edge_prev && ew.prev_in) prev = from_prev;
     const unsigned lo = __byte_perm(prev, Y.x, 0x5410), hi = __byte_perm(Y.x, Y.y, 0x5432);
-    if (!xl.edge_prev || prev_in) {
+    if (!xl.edge_prev || ew.prev_in) {
       *reinterpret_cast<uint2*>(p + i0) = make_uint2(lo, hi);
     } else {
       u[i0 + 1] = (unsigned short)(Y.x & 0xffffu);
       *reinterpret_cast<unsigned*>(p + i0 + 2) = hi;
     }
-    if (xl.edge_next && !next_in) u[i_next] = (unsigned short)(Y.y >> 16);
+    if (xl.edge_next && !ew.next_in) {
+      unsigned v = Y.y >> 16;
+      if (at.last()) v = at.cells == 1 ? Y.x : (at.cells == 2 ? Y.x >> 16 : Y.y);
+      u[at.i_next] = (unsigned short)(v & 0xffffu);
+    }
   } else {  // cell i0+m -> element i0+m-1
     unsigned next = __shfl_sync(0xffffffffu, Y.x & 0xffffu, xl.src_next);  // cell i0+4 of the lane after
-    if (xl.edge_next && next_in) next = from_next;
+    if (xl.edge_next && ew.next_in) next = from_next;
     const unsigned lo = __byte_perm(Y.x, Y.y, 0x5432), hi = __byte_perm(Y.y, next, 0x5432);
-    if (!xl.edge_next || next_in) {
+    if (!xl.edge_next || ew.next_in) {
       *reinterpret_cast<uint2*>(p + i0) = make_uint2(lo, hi);
+    } else if (at.last()) {
+      // cells 1.. go one element back; the row's last element is its first cell's
+      if (at.cells > 1) u[i0] = (unsigned short)(Y.x >> 16);
+      if (at.cells > 2) u[i0 + 1] = (unsigned short)(Y.y & 0xffffu);
     } else {
       *reinterpret_cast<unsigned*>(p + i0) = lo;
       u[i0 + 2] = (unsigned short)(Y.y >> 16);
     }
-    if (xl.edge_prev && !prev_in) u[i_prev] = (unsigned short)(Y.x & 0xffffu);
+    if (xl.edge_prev && !ew.prev_in) u[at.i_prev] = (unsigned short)(Y.x & 0xffffu);
   }
 }
 
-template <bool ODD, bool LES>
-__global__ void __launch_bounds__(128, 5) k_aa_f16v(Pops<__half> a, Geo g, StepK K, int log_tpr) {
-  const int tpr = 1 << log_tpr;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j0 = t >> log_tpr, pos = t & (tpr - 1);
+template <bool ODD, bool LES, bool FLAT>
+__global__ void __launch_bounds__(128, 5) k_aa_f16v(Pops<__half> a, Geo g, StepK K, int rows) {
+  const VecPlace<4, FLAT> at(g, rows);
   const int k = blockIdx.y;
-  const bool valid = j0 < g.ny;  // whole warps: ny*tpr is a multiple of 32
+  const bool valid = at.valid;  // whole warps unless FLAT
   if (!ODD && !valid) return;
-  const int j = valid ? j0 : 0;  // an idle warp of the odd step only reaches its barrier
-  const XLanes xl(tpr, pos, threadIdx.x & 31);
-  const int i0 = pos * 4;
+  const int j = at.j;  // idle threads of the odd step only reach its barrier
+  const XLanes xl(at, threadIdx.x & 31);
+  const int i0 = at.i0;
   const int jm = j == 0 ? g.ny - 1 : j - 1, jp = j == g.ny - 1 ? 0 : j + 1;
   const int km = k == 0 ? g.nz - 1 : k - 1, kp = k == g.nz - 1 ? 0 : k + 1;
-  const int i_prev = pos == 0 ? g.nx - 1 : i0 - 1;
-  const int i_next = pos == tpr - 1 ? 0 : i0 + 4;
   auto row = [&](int dy, int dz) {  // row offset of (j + dy, k + dz), dy, dz in {-1, 0, 1}
     const int jj = dy > 0 ? jp : (dy < 0 ? jm : j);
     const int kk = dz > 0 ? kp : (dz < 0 ? km : k);
     return g.sx * (jj + g.ny * kk);
   };
   uint2 Y[Q];
-  if (ODD && !valid) {
+  if (ODD && !FLAT && !valid) {
 #pragma unroll
     for (int q = 0; q < Q; ++q) Y[q] = make_uint2(0u, 0u);
   } else if (ODD) {
@@ -411,36 +413,25 @@ __global__ void __launch_bounds__(128, 5) k_aa_f16v(Pops<__half> a, Geo g, StepK
       const __half* p = a.p[oppq(q)] + row(-cyq(q), -czq(q));
       Y[q] = __ldg(reinterpret_cast<const uint2*>(p + i0));
       E[q] = 0;
-      if (cxq(q) > 0 && xl.edge_prev) E[q] = ldg_u16(p + i_prev);
-      if (cxq(q) < 0 && xl.edge_next) E[q] = ldg_u16(p + i_next);
+      if (cxq(q) > 0 && xl.edge_prev) E[q] = ldg_u16(p + at.i_prev);
+      if (cxq(q) < 0 && xl.edge_next) E[q] = ldg_u16(p + at.i_next);
     }
+    if (at.last()) wrap_last(Y, E, at.cells);
     shift_rows(Y, E, xl);
   } else {
 #pragma unroll
     for (int q = 0; q < Q; ++q) Y[q] = __ldg(reinterpret_cast<const uint2*>(a.p[q] + row(0, 0) + i0));
   }
-  if (valid) collide4_f16<LES>(Y, K);
+  if (FLAT || valid) collide4_f16<LES>(Y, K);
   // odd step: the warps' crossing values (cx > 0 populations: the last
   // lane's last cell; cx < 0: the first lane's first cell) through shared
   // memory; the barrier also orders every warp's loads before any warp's
   // stores of its neighbours' crossing elements
   __shared__ unsigned xs_last[ODD ? 4 : 1][5], xs_first[ODD ? 4 : 1][5];
-  bool prev_in = false, next_in = false;
-  int wprev = 0, wnext = 0;
+  const EdgeWarps ew(at);
   if (ODD) {
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (tpr >= 32) {
-      const int nw = tpr >> 5, r = pos >> 5;  // warps per row, this warp's place in its row
-      if (nw <= 4) {  // the whole row in this block
-        prev_in = next_in = true;
-        wprev = w - r + (r + nw - 1) % nw;
-        wnext = w - r + (r + 1) % nw;
-      } else {
-        prev_in = w > 0;
-        next_in = w < 3;
-        wprev = w - 1;
-        wnext = w + 1;
-      }
+    if (ew.any) {
       if (valid && lane == 31) {
 #pragma unroll
         for (int q = 0; q < 5; ++q) xs_last[w][q] = Y[q].y >> 16;
@@ -467,9 +458,9 @@ __global__ void __launch_bounds__(128, 5) k_aa_f16v(Pops<__half> a, Geo g, StepK
     if (!ODD) {
       *reinterpret_cast<uint2*>(a.p[oppq(q)] + row(0, 0) + i0) = Y[q];
     } else {
-      const unsigned fp = cxq(q) > 0 && xl.edge_prev && prev_in ? xs_last[wprev][q] : 0u;
-      const unsigned fn = cxq(q) < 0 && xl.edge_next && next_in ? xs_first[wnext][q - 9] : 0u;
-      shift_out(Y[q], cxq(q), a.p[q] + row_out(cyq(q), czq(q)), i0, i_prev, i_next, xl, prev_in, next_in, fp, fn);
+      const unsigned fp = cxq(q) > 0 && xl.edge_prev && ew.prev_in ? xs_last[ew.wprev][q] : 0u;
+      const unsigned fn = cxq(q) < 0 && xl.edge_next && ew.next_in ? xs_first[ew.wnext][q - 9] : 0u;
+      shift_out(Y[q], cxq(q), a.p[q] + row_out(cyq(q), czq(q)), at, xl, ew, fp, fn);
     }
   }
 }
@@ -507,63 +498,60 @@ __device__ __forceinline__ void shift_rows8(uint4 (&Y)[Q], const unsigned short 
 // i0+m goes to element i0+m+cx; the aligned chunk i0..i0+7 is completed with
 // the neighbouring lane's crossing value, and at block boundaries the edge
 // lanes store their part with 2-, 4- and 8-byte stores.
-__device__ __forceinline__ void shift_out8(uint4 Y, int cx, __half* p, int i0, int i_prev, int i_next,
-                                           const XLanes& xl, bool prev_in, bool next_in, unsigned from_prev,
-                                           unsigned from_next) {
+template <bool FLAT>
+__device__ __forceinline__ void shift_out8(uint4 Y, int cx, __half* p, const VecPlace<8, FLAT>& at, const XLanes& xl,
+                                           const EdgeWarps& ew, unsigned from_prev, unsigned from_next) {
+  const int i0 = at.i0;
   unsigned short* u = reinterpret_cast<unsigned short*>(p);
   if (cx == 0) {
     *reinterpret_cast<uint4*>(p + i0) = Y;
   } else if (cx > 0) {  // cell i0+m -> element i0+m+1
     unsigned prev = __shfl_sync(0xffffffffu, Y.w >> 16, xl.src_prev);  // cell i0-1 of the lane before
-    if (xl.edge_prev && prev_in) prev = from_prev;
+    if (xl.edge_prev && ew.prev_in) prev = from_prev;
     const uint4 c = make_uint4(__byte_perm(prev, Y.x, 0x5410), __byte_perm(Y.x, Y.y, 0x5432),
                                __byte_perm(Y.y, Y.z, 0x5432), __byte_perm(Y.z, Y.w, 0x5432));
-    if (!xl.edge_prev || prev_in) {
+    if (!xl.edge_prev || ew.prev_in) {
       *reinterpret_cast<uint4*>(p + i0) = c;
     } else {
       u[i0 + 1] = (unsigned short)(Y.x & 0xffffu);
       *reinterpret_cast<unsigned*>(p + i0 + 2) = c.y;
       *reinterpret_cast<uint2*>(p + i0 + 4) = make_uint2(c.z, c.w);
     }
-    if (xl.edge_next && !next_in) u[i_next] = (unsigned short)(Y.w >> 16);
+    if (xl.edge_next && !ew.next_in) u[at.i_next] = (unsigned short)(Y.w >> 16);
   } else {  // cell i0+m -> element i0+m-1
     unsigned next = __shfl_sync(0xffffffffu, Y.x & 0xffffu, xl.src_next);  // cell i0+8 of the lane after
-    if (xl.edge_next && next_in) next = from_next;
+    if (xl.edge_next && ew.next_in) next = from_next;
     const uint4 c = make_uint4(__byte_perm(Y.x, Y.y, 0x5432), __byte_perm(Y.y, Y.z, 0x5432),
                                __byte_perm(Y.z, Y.w, 0x5432), __byte_perm(Y.w, next, 0x5432));
-    if (!xl.edge_next || next_in) {
+    if (!xl.edge_next || ew.next_in) {
       *reinterpret_cast<uint4*>(p + i0) = c;
     } else {
       *reinterpret_cast<uint2*>(p + i0) = make_uint2(c.x, c.y);
       *reinterpret_cast<unsigned*>(p + i0 + 4) = c.z;
       u[i0 + 6] = (unsigned short)(Y.w >> 16);
     }
-    if (xl.edge_prev && !prev_in) u[i_prev] = (unsigned short)(Y.x & 0xffffu);
+    if (xl.edge_prev && !ew.prev_in) u[at.i_prev] = (unsigned short)(Y.x & 0xffffu);
   }
 }
 
-template <bool ODD>
-__global__ void __launch_bounds__(128, 4) k_aa_f16w(Pops<__half> a, Geo g, StepK K, int log_tpr) {
-  const int tpr = 1 << log_tpr;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j0 = t >> log_tpr, pos = t & (tpr - 1);
+template <bool ODD, bool FLAT>
+__global__ void __launch_bounds__(128, 4) k_aa_f16w(Pops<__half> a, Geo g, StepK K, int rows) {
+  const VecPlace<8, FLAT> at(g, rows);
   const int k = blockIdx.y;
-  const bool valid = j0 < g.ny;  // whole warps: ny*tpr is a multiple of 32
+  const bool valid = at.valid;  // whole warps unless FLAT
   if (!ODD && !valid) return;
-  const int j = valid ? j0 : 0;  // an idle warp of the odd step only reaches its barrier
-  const XLanes xl(tpr, pos, threadIdx.x & 31);
-  const int i0 = pos * 8;
+  const int j = at.j;  // idle threads of the odd step only reach its barrier
+  const XLanes xl(at, threadIdx.x & 31);
+  const int i0 = at.i0;
   const int jm = j == 0 ? g.ny - 1 : j - 1, jp = j == g.ny - 1 ? 0 : j + 1;
   const int km = k == 0 ? g.nz - 1 : k - 1, kp = k == g.nz - 1 ? 0 : k + 1;
-  const int i_prev = pos == 0 ? g.nx - 1 : i0 - 1;
-  const int i_next = pos == tpr - 1 ? 0 : i0 + 8;
   auto row = [&](int dy, int dz) {
     const int jj = dy > 0 ? jp : (dy < 0 ? jm : j);
     const int kk = dz > 0 ? kp : (dz < 0 ? km : k);
     return g.sx * (jj + g.ny * kk);
   };
   uint4 Y[Q];
-  if (ODD && !valid) {
+  if (ODD && !FLAT && !valid) {
 #pragma unroll
     for (int q = 0; q < Q; ++q) Y[q] = make_uint4(0u, 0u, 0u, 0u);
   } else if (ODD) {
@@ -573,15 +561,15 @@ __global__ void __launch_bounds__(128, 4) k_aa_f16w(Pops<__half> a, Geo g, StepK
       const __half* p = a.p[oppq(q)] + row(-cyq(q), -czq(q));
       Y[q] = __ldg(reinterpret_cast<const uint4*>(p + i0));
       E[q] = 0;
-      if (cxq(q) > 0 && xl.edge_prev) E[q] = ldg_u16(p + i_prev);
-      if (cxq(q) < 0 && xl.edge_next) E[q] = ldg_u16(p + i_next);
+      if (cxq(q) > 0 && xl.edge_prev) E[q] = ldg_u16(p + at.i_prev);
+      if (cxq(q) < 0 && xl.edge_next) E[q] = ldg_u16(p + at.i_next);
     }
     shift_rows8(Y, E, xl);
   } else {
 #pragma unroll
     for (int q = 0; q < Q; ++q) Y[q] = __ldg(reinterpret_cast<const uint4*>(a.p[q] + row(0, 0) + i0));
   }
-  if (valid) {
+  if (FLAT || valid) {
     uint2 L[Q], H[Q];
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
@@ -594,22 +582,10 @@ __global__ void __launch_bounds__(128, 4) k_aa_f16w(Pops<__half> a, Geo g, StepK
     for (int q = 0; q < Q; ++q) Y[q] = make_uint4(L[q].x, L[q].y, H[q].x, H[q].y);
   }
   __shared__ unsigned xs_last[ODD ? 4 : 1][5], xs_first[ODD ? 4 : 1][5];
-  bool prev_in = false, next_in = false;
-  int wprev = 0, wnext = 0;
+  const EdgeWarps ew(at);
   if (ODD) {
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (tpr >= 32) {
-      const int nw = tpr >> 5, r = pos >> 5;
-      if (nw <= 4) {
-        prev_in = next_in = true;
-        wprev = w - r + (r + nw - 1) % nw;
-        wnext = w - r + (r + 1) % nw;
-      } else {
-        prev_in = w > 0;
-        next_in = w < 3;
-        wprev = w - 1;
-        wnext = w + 1;
-      }
+    if (ew.any) {
       if (valid && lane == 31) {
 #pragma unroll
         for (int q = 0; q < 5; ++q) xs_last[w][q] = Y[q].w >> 16;
@@ -636,9 +612,9 @@ __global__ void __launch_bounds__(128, 4) k_aa_f16w(Pops<__half> a, Geo g, StepK
     if (!ODD) {
       *reinterpret_cast<uint4*>(a.p[oppq(q)] + row(0, 0) + i0) = Y[q];
     } else {
-      const unsigned fp = cxq(q) > 0 && xl.edge_prev && prev_in ? xs_last[wprev][q] : 0u;
-      const unsigned fn = cxq(q) < 0 && xl.edge_next && next_in ? xs_first[wnext][q - 9] : 0u;
-      shift_out8(Y[q], cxq(q), a.p[q] + row_out(cyq(q), czq(q)), i0, i_prev, i_next, xl, prev_in, next_in, fp, fn);
+      const unsigned fp = cxq(q) > 0 && xl.edge_prev && ew.prev_in ? xs_last[ew.wprev][q] : 0u;
+      const unsigned fn = cxq(q) < 0 && xl.edge_next && ew.next_in ? xs_first[ew.wnext][q - 9] : 0u;
+      shift_out8(Y[q], cxq(q), a.p[q] + row_out(cyq(q), czq(q)), at, xl, ew, fp, fn);
     }
   }
 }
@@ -646,23 +622,24 @@ __global__ void __launch_bounds__(128, 4) k_aa_f16w(Pops<__half> a, Geo g, StepK
 // Store side of the FP32 odd step: cells i0, i0+1 go to elements i0 + cx,
 // i0 + 1 + cx of row p, stored as the aligned chunk (i0, i0+1) completed with
 // the neighbouring lane's crossing value, as shift_out does for FP16.
-__device__ __forceinline__ void shift_out_f32(float2 Y, int cx, float* p, int i0, int i_prev, int i_next,
-                                              const XLanes& xl, bool prev_in, bool next_in, float from_prev,
-                                              float from_next) {
+template <bool FLAT>
+__device__ __forceinline__ void shift_out_f32(float2 Y, int cx, float* p, const VecPlace<2, FLAT>& at, const XLanes& xl,
+                                              const EdgeWarps& ew, float from_prev, float from_next) {
+  const int i0 = at.i0;
   if (cx == 0) {
     *reinterpret_cast<float2*>(p + i0) = Y;
   } else if (cx > 0) {  // cell i0+m -> element i0+m+1
     float prev = __shfl_sync(0xffffffffu, Y.y, xl.src_prev);  // cell i0-1 of the lane before
-    if (xl.edge_prev && prev_in) prev = from_prev;
-    if (!xl.edge_prev || prev_in) *reinterpret_cast<float2*>(p + i0) = make_float2(prev, Y.x);
+    if (xl.edge_prev && ew.prev_in) prev = from_prev;
+    if (!xl.edge_prev || ew.prev_in) *reinterpret_cast<float2*>(p + i0) = make_float2(prev, Y.x);
     else p[i0 + 1] = Y.x;
-    if (xl.edge_next && !next_in) p[i_next] = Y.y;
+    if (xl.edge_next && !ew.next_in) p[at.i_next] = at.last() ? Y.x : Y.y;
   } else {  // cell i0+m -> element i0+m-1
     float next = __shfl_sync(0xffffffffu, Y.x, xl.src_next);  // cell i0+2 of the lane after
-    if (xl.edge_next && next_in) next = from_next;
-    if (!xl.edge_next || next_in) *reinterpret_cast<float2*>(p + i0) = make_float2(Y.y, next);
-    else p[i0] = Y.y;
-    if (xl.edge_prev && !prev_in) p[i_prev] = Y.x;
+    if (xl.edge_next && ew.next_in) next = from_next;
+    if (!xl.edge_next || ew.next_in) *reinterpret_cast<float2*>(p + i0) = make_float2(Y.y, next);
+    else if (!at.last()) p[i0] = Y.y;
+    if (xl.edge_prev && !ew.prev_in) p[at.i_prev] = Y.x;
   }
 }
 
@@ -672,28 +649,24 @@ __device__ __forceinline__ void shift_out_f32(float2 Y, int cx, float* p, int i0
 // order) on each cell, so the results are those of k_aa<F32, ODD>. The same
 // ownership argument keeps the in-place update race-free. 95 registers (87
 // for the Smagorinsky even step), no spills.
-template <bool ODD, bool LES>
-__global__ void __launch_bounds__(128, 5) k_aa_f32v(Pops<float> a, Geo g, StepK K, int log_tpr) {
-  const int tpr = 1 << log_tpr;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j0 = t >> log_tpr, pos = t & (tpr - 1);
+template <bool ODD, bool LES, bool FLAT>
+__global__ void __launch_bounds__(128, 5) k_aa_f32v(Pops<float> a, Geo g, StepK K, int rows) {
+  const VecPlace<2, FLAT> at(g, rows);
   const int k = blockIdx.y;
-  const bool valid = j0 < g.ny;  // whole warps: ny*tpr is a multiple of 32
+  const bool valid = at.valid;  // whole warps unless FLAT
   if (!ODD && !valid) return;
-  const int j = valid ? j0 : 0;  // an idle warp of the odd step only reaches its barrier
-  const XLanes xl(tpr, pos, threadIdx.x & 31);
-  const int i0 = pos * 2;
+  const int j = at.j;  // idle threads of the odd step only reach its barrier
+  const XLanes xl(at, threadIdx.x & 31);
+  const int i0 = at.i0;
   const int jm = j == 0 ? g.ny - 1 : j - 1, jp = j == g.ny - 1 ? 0 : j + 1;
   const int km = k == 0 ? g.nz - 1 : k - 1, kp = k == g.nz - 1 ? 0 : k + 1;
-  const int i_prev = pos == 0 ? g.nx - 1 : i0 - 1;
-  const int i_next = pos == tpr - 1 ? 0 : i0 + 2;
   auto row = [&](int dy, int dz) {  // row offset of (j + dy, k + dz), dy, dz in {-1, 0, 1}
     const int jj = dy > 0 ? jp : (dy < 0 ? jm : j);
     const int kk = dz > 0 ? kp : (dz < 0 ? km : k);
     return g.sx * (jj + g.ny * kk);
   };
   float2 Y[Q];
-  if (ODD && !valid) {
+  if (ODD && !FLAT && !valid) {
 #pragma unroll
     for (int q = 0; q < Q; ++q) Y[q] = make_float2(0.f, 0.f);
   } else if (ODD) {
@@ -703,15 +676,16 @@ __global__ void __launch_bounds__(128, 5) k_aa_f32v(Pops<float> a, Geo g, StepK 
       const float* p = a.p[oppq(q)] + row(-cyq(q), -czq(q));
       Y[q] = __ldg(reinterpret_cast<const float2*>(p + i0));
       E[q] = 0.f;
-      if (cxq(q) > 0 && xl.edge_prev) E[q] = __ldg(p + i_prev);
-      if (cxq(q) < 0 && xl.edge_next) E[q] = __ldg(p + i_next);
+      if (cxq(q) > 0 && xl.edge_prev) E[q] = __ldg(p + at.i_prev);
+      if (cxq(q) < 0 && xl.edge_next) E[q] = __ldg(p + at.i_next);
     }
+    if (at.last()) wrap_last(Y, E, at.cells);
     shift_rows_f32(Y, E, xl);
   } else {
 #pragma unroll
     for (int q = 0; q < Q; ++q) Y[q] = __ldg(reinterpret_cast<const float2*>(a.p[q] + row(0, 0) + i0));
   }
-  if (valid) {
+  if (FLAT || valid) {
 #pragma unroll
     for (int m = 0; m < 2; ++m) {
       float s[Q];
@@ -726,22 +700,10 @@ __global__ void __launch_bounds__(128, 5) k_aa_f32v(Pops<float> a, Geo g, StepK 
     }
   }
   __shared__ float xs_last[ODD ? 4 : 1][5], xs_first[ODD ? 4 : 1][5];
-  bool prev_in = false, next_in = false;
-  int wprev = 0, wnext = 0;
+  const EdgeWarps ew(at);
   if (ODD) {
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (tpr >= 32) {
-      const int nw = tpr >> 5, r = pos >> 5;  // warps per row, this warp's place in its row
-      if (nw <= 4) {  // the whole row in this block
-        prev_in = next_in = true;
-        wprev = w - r + (r + nw - 1) % nw;
-        wnext = w - r + (r + 1) % nw;
-      } else {
-        prev_in = w > 0;
-        next_in = w < 3;
-        wprev = w - 1;
-        wnext = w + 1;
-      }
+    if (ew.any) {
       if (valid && lane == 31) {
 #pragma unroll
         for (int q = 0; q < 5; ++q) xs_last[w][q] = Y[q].y;
@@ -768,10 +730,9 @@ __global__ void __launch_bounds__(128, 5) k_aa_f32v(Pops<float> a, Geo g, StepK 
     if (!ODD) {
       *reinterpret_cast<float2*>(a.p[oppq(q)] + row(0, 0) + i0) = Y[q];
     } else {
-      const float fp = cxq(q) > 0 && xl.edge_prev && prev_in ? xs_last[wprev][q] : 0.f;
-      const float fn = cxq(q) < 0 && xl.edge_next && next_in ? xs_first[wnext][q - 9] : 0.f;
-      shift_out_f32(Y[q], cxq(q), a.p[q] + row_out(cyq(q), czq(q)), i0, i_prev, i_next, xl, prev_in, next_in, fp,
-                    fn);
+      const float fp = cxq(q) > 0 && xl.edge_prev && ew.prev_in ? xs_last[ew.wprev][q] : 0.f;
+      const float fn = cxq(q) < 0 && xl.edge_next && ew.next_in ? xs_first[ew.wnext][q - 9] : 0.f;
+      shift_out_f32(Y[q], cxq(q), a.p[q] + row_out(cyq(q), czq(q)), at, xl, ew, fp, fn);
     }
   }
 }
@@ -781,55 +742,52 @@ __global__ void __launch_bounds__(128, 5) k_aa_f32v(Pops<float> a, Geo g, StepK 
 // its per-thread x-crossing work covers twice the cells, as k_aa_f16w does
 // for FP16. F32::cell's arithmetic on each cell: the results of k_aa<F32>.
 // 125 registers (127 with the Smagorinsky collision), 4 blocks/SM, no spills.
-__device__ __forceinline__ void shift_out4_f32(float4 Y, int cx, float* p, int i0, int i_prev, int i_next,
-                                               const XLanes& xl, bool prev_in, bool next_in, float from_prev,
-                                               float from_next) {
+template <bool FLAT>
+__device__ __forceinline__ void shift_out4_f32(float4 Y, int cx, float* p, const VecPlace<4, FLAT>& at, const XLanes& xl,
+                                               const EdgeWarps& ew, float from_prev, float from_next) {
+  const int i0 = at.i0;
   if (cx == 0) {
     *reinterpret_cast<float4*>(p + i0) = Y;
   } else if (cx > 0) {  // cell i0+m -> element i0+m+1
     float prev = __shfl_sync(0xffffffffu, Y.w, xl.src_prev);  // cell i0-1 of the lane before
-    if (xl.edge_prev && prev_in) prev = from_prev;
-    if (!xl.edge_prev || prev_in) {
+    if (xl.edge_prev && ew.prev_in) prev = from_prev;
+    if (!xl.edge_prev || ew.prev_in) {
       *reinterpret_cast<float4*>(p + i0) = make_float4(prev, Y.x, Y.y, Y.z);
     } else {
       p[i0 + 1] = Y.x;
       *reinterpret_cast<float2*>(p + i0 + 2) = make_float2(Y.y, Y.z);
     }
-    if (xl.edge_next && !next_in) p[i_next] = Y.w;
+    if (xl.edge_next && !ew.next_in) p[at.i_next] = Y.w;
   } else {  // cell i0+m -> element i0+m-1
     float next = __shfl_sync(0xffffffffu, Y.x, xl.src_next);  // cell i0+4 of the lane after
-    if (xl.edge_next && next_in) next = from_next;
-    if (!xl.edge_next || next_in) {
+    if (xl.edge_next && ew.next_in) next = from_next;
+    if (!xl.edge_next || ew.next_in) {
       *reinterpret_cast<float4*>(p + i0) = make_float4(Y.y, Y.z, Y.w, next);
     } else {
       *reinterpret_cast<float2*>(p + i0) = make_float2(Y.y, Y.z);
       p[i0 + 2] = Y.w;
     }
-    if (xl.edge_prev && !prev_in) p[i_prev] = Y.x;
+    if (xl.edge_prev && !ew.prev_in) p[at.i_prev] = Y.x;
   }
 }
 
-template <bool LES = false>
-__global__ void __launch_bounds__(128, 4) k_aa_f32w(Pops<float> a, Geo g, StepK K, int log_tpr) {
-  const int tpr = 1 << log_tpr;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j0 = t >> log_tpr, pos = t & (tpr - 1);
+template <bool LES, bool FLAT>
+__global__ void __launch_bounds__(128, 4) k_aa_f32w(Pops<float> a, Geo g, StepK K, int rows) {
+  const VecPlace<4, FLAT> at(g, rows);
   const int k = blockIdx.y;
-  const bool valid = j0 < g.ny;  // whole warps: ny*tpr is a multiple of 32
-  const int j = valid ? j0 : 0;  // an idle warp only reaches its barrier
-  const XLanes xl(tpr, pos, threadIdx.x & 31);
-  const int i0 = pos * 4;
+  const bool valid = at.valid;  // whole warps unless FLAT
+  const int j = at.j;  // idle threads of the odd step only reach its barrier
+  const XLanes xl(at, threadIdx.x & 31);
+  const int i0 = at.i0;
   const int jm = j == 0 ? g.ny - 1 : j - 1, jp = j == g.ny - 1 ? 0 : j + 1;
   const int km = k == 0 ? g.nz - 1 : k - 1, kp = k == g.nz - 1 ? 0 : k + 1;
-  const int i_prev = pos == 0 ? g.nx - 1 : i0 - 1;
-  const int i_next = pos == tpr - 1 ? 0 : i0 + 4;
   auto row = [&](int dy, int dz) {
     const int jj = dy > 0 ? jp : (dy < 0 ? jm : j);
     const int kk = dz > 0 ? kp : (dz < 0 ? km : k);
     return g.sx * (jj + g.ny * kk);
   };
   float4 Y[Q];
-  if (!valid) {
+  if (!FLAT && !valid) {
 #pragma unroll
     for (int q = 0; q < Q; ++q) Y[q] = make_float4(0.f, 0.f, 0.f, 0.f);
   } else {
@@ -839,8 +797,8 @@ __global__ void __launch_bounds__(128, 4) k_aa_f32w(Pops<float> a, Geo g, StepK 
       const float* p = a.p[oppq(q)] + row(-cyq(q), -czq(q));
       Y[q] = __ldg(reinterpret_cast<const float4*>(p + i0));
       E[q] = 0.f;
-      if (cxq(q) > 0 && xl.edge_prev) E[q] = __ldg(p + i_prev);
-      if (cxq(q) < 0 && xl.edge_next) E[q] = __ldg(p + i_next);
+      if (cxq(q) > 0 && xl.edge_prev) E[q] = __ldg(p + at.i_prev);
+      if (cxq(q) < 0 && xl.edge_next) E[q] = __ldg(p + at.i_next);
     }
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
@@ -871,21 +829,9 @@ __global__ void __launch_bounds__(128, 4) k_aa_f32w(Pops<float> a, Geo g, StepK 
     }
   }
   __shared__ float xs_last[4][5], xs_first[4][5];
-  bool prev_in = false, next_in = false;
-  int wprev = 0, wnext = 0;
+  const EdgeWarps ew(at);
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (tpr >= 32) {
-    const int nw = tpr >> 5, r = pos >> 5;  // warps per row, this warp's place in its row
-    if (nw <= 4) {  // the whole row in this block
-      prev_in = next_in = true;
-      wprev = w - r + (r + nw - 1) % nw;
-      wnext = w - r + (r + 1) % nw;
-    } else {
-      prev_in = w > 0;
-      next_in = w < 3;
-      wprev = w - 1;
-      wnext = w + 1;
-    }
+  if (ew.any) {
     if (valid && lane == 31) {
 #pragma unroll
       for (int q = 0; q < 5; ++q) xs_last[w][q] = Y[q].w;
@@ -908,9 +854,9 @@ __global__ void __launch_bounds__(128, 4) k_aa_f32w(Pops<float> a, Geo g, StepK 
   };
 #pragma unroll
   for (int q = 0; q < Q; ++q) {
-    const float fp = cxq(q) > 0 && xl.edge_prev && prev_in ? xs_last[wprev][q] : 0.f;
-    const float fn = cxq(q) < 0 && xl.edge_next && next_in ? xs_first[wnext][q - 9] : 0.f;
-    shift_out4_f32(Y[q], cxq(q), a.p[q] + row_out(cyq(q), czq(q)), i0, i_prev, i_next, xl, prev_in, next_in, fp, fn);
+    const float fp = cxq(q) > 0 && xl.edge_prev && ew.prev_in ? xs_last[ew.wprev][q] : 0.f;
+    const float fn = cxq(q) < 0 && xl.edge_next && ew.next_in ? xs_first[ew.wnext][q - 9] : 0.f;
+    shift_out4_f32(Y[q], cxq(q), a.p[q] + row_out(cyq(q), czq(q)), at, xl, ew, fp, fn);
   }
 }
 
@@ -1615,10 +1561,13 @@ StepK make_stepk(int form, double omega, double scale, double les_cs) {
   return k;
 }
 
-// Grid of the several-cells-per-thread kernels: 128-thread blocks over the
-// ny * 2^log_tpr threads of a plane, `planes` planes.
-static dim3 vec_grid(const Geo& g, int log_tpr, int planes) {
-  return dim3((unsigned)((((long long)g.ny << log_tpr) + 127) / 128), (unsigned)planes);
+// Launches a several-cells-per-thread kernel (its aligned and its flat
+// instantiation) in 128-thread blocks over the threads of `planes` planes.
+template <class KA, class KF, class... Args>
+static void launch_vec(KA aligned, KF flat, const Geo& g, const VecRows& r, int planes, cudaStream_t st, Args... args) {
+  const dim3 grid((unsigned)(((long long)g.ny * r.tpr + 127) / 128), (unsigned)planes);
+  if (r.flat) flat<<<grid, 128, 0, st>>>(args...);
+  else aligned<<<grid, 128, 0, st>>>(args...);
 }
 
 template <class F>
@@ -1628,28 +1577,33 @@ static cudaError_t two_impl(const Lattice& s, const Lattice& d, const StepK& K, 
   Pops<S> pd = pops_of<S>(d);
   pd.p[Q - 1] = (S*)s.p[Q - 1];  // pop 19 in place (SRC/col_MC.F90:351)
   Shape sh = cell_shape(s.g);
-  // FP32: two cells per thread where the box fits it (automatic or 2): on
-  // B200 at 256^3, 43.7 GLUPS against 42.0 with one cell per thread, the
-  // Smagorinsky step 43.5 against 40.7
-  const int lt2 = F::id == FORM_F32 && (variant == 0 || variant == 2) ? vec_log_tpr(s.g, 2) : -1;
-  if (lt2 >= 0) {
+  const long long cells = (long long)s.g.nx * s.g.ny * s.g.nz;
+  // FP32: two cells per thread (automatic or 2): on B200 at 256^3, 43.7 GLUPS
+  // against 42.0 with one cell per thread, the Smagorinsky step 43.5 against
+  // 40.7; rows of no power of two: 180^3 39.0 against 34.4
+  const bool big = cells >= VEC_MIN_TWO;
+  if (F::id == FORM_F32 && (variant == 2 || (variant == 0 && big))) {
     Pops<float> pf = pops_of<float>(d);
     pf.p[Q - 1] = (float*)s.p[Q - 1];
-    const dim3 grid = vec_grid(s.g, lt2, s.g.nz);
-    if (K.les) k_two_f32v<true><<<grid, 128, 0, st>>>(pops_of<const float>(s), pf, s.g, K, lt2, 0);
-    else k_two_f32v<false><<<grid, 128, 0, st>>>(pops_of<const float>(s), pf, s.g, K, lt2, 0);
+    const VecRows r(s.g, 2, true);
+    if (K.les) launch_vec(k_two_f32v<true, false>, k_two_f32v<true, true>, s.g, r, s.g.nz, st, pops_of<const float>(s), pf, s.g, K, r.arg, 0);
+    else launch_vec(k_two_f32v<false, false>, k_two_f32v<false, true>, s.g, r, s.g.nz, st, pops_of<const float>(s), pf, s.g, K, r.arg, 0);
     return cudaGetLastError();
   }
-  if (K.les) {  // the Smagorinsky collision: one cell per thread, FP16 four where the box fits
-    const int lt = F::id == FORM_F16 && (variant == 0 || variant == 4) ? vec_log_tpr(s.g, 4) : -1;
-    if (lt >= 0) {
-      Pops<__half> ph = pops_of<__half>(d);
-      ph.p[Q - 1] = (__half*)s.p[Q - 1];
-      const dim3 grid = vec_grid(s.g, lt, s.g.nz);
-      k_two_f16v<true><<<grid, 128, 0, st>>>(pops_of<const __half>(s), ph, s.g, K, lt, 0);
-    } else {
-      k_two<F, true><<<sh.grid, sh.block, 0, st>>>(ps, pd, s.g, K);
-    }
+  // FP16: four cells per thread (automatic or 4; the Smagorinsky step too), the
+  // fastest measured on B200 at 256^3 (76.6 GLUPS against 64.0 with one, 62.7
+  // with two and 44.6 for the row pipeline); rows of no power of two: 201 x 163 x 117 71.9
+  // against 49.8, 180^3 74.3 against 51.3
+  if (F::id == FORM_F16 && (variant == 4 || (variant == 0 && big))) {
+    Pops<__half> ph = pops_of<__half>(d);
+    ph.p[Q - 1] = (__half*)s.p[Q - 1];
+    const VecRows r(s.g, 4, true);
+    if (K.les) launch_vec(k_two_f16v<true, false>, k_two_f16v<true, true>, s.g, r, s.g.nz, st, pops_of<const __half>(s), ph, s.g, K, r.arg, 0);
+    else launch_vec(k_two_f16v<false, false>, k_two_f16v<false, true>, s.g, r, s.g.nz, st, pops_of<const __half>(s), ph, s.g, K, r.arg, 0);
+    return cudaGetLastError();
+  }
+  if (K.les) {  // the other choices run the Smagorinsky collision on one cell per thread
+    k_two<F, true><<<sh.grid, sh.block, 0, st>>>(ps, pd, s.g, K);
     return cudaGetLastError();
   }
   if (variant == 8) {
@@ -1657,20 +1611,13 @@ static cudaError_t two_impl(const Lattice& s, const Lattice& d, const StepK& K, 
     cudaError_t e = launch_rows(s, d, ROW_TWO, K, st, &launched);
     if (e != cudaSuccess || launched) return e;
   }
-  // automatic choice (variant 0): one cell per thread for FP64, two for FP32
-  // (above), four cells per thread for FP16 where the box fits it - the fastest measured on
-  // B200 at 256^3 (FP16: 76.6 GLUPS with four cells per thread against 64.0
-  // with one, 62.7 with two and 44.6 for the row pipeline)
-  if (F::id == FORM_F16 && (variant == 2 || variant == 4 || variant == 0)) {
-    const int V = variant == 0 ? 4 : variant;
-    const int lt = vec_log_tpr(s.g, V);
-    if (lt >= 0) {
-      const long long threads = (long long)s.g.ny << lt;
-      dim3 grid((unsigned)((threads + (V == 4 ? 127 : 255)) / (V == 4 ? 128 : 256)), s.g.nz);
+  if (F::id == FORM_F16 && variant == 2) {
+    const VecRows r(s.g, 2, true);
+    if (!r.flat) {
       Pops<__half> ph = pops_of<__half>(d);
       ph.p[Q - 1] = (__half*)s.p[Q - 1];
-      if (V == 4) k_two_f16v<false><<<grid, 128, 0, st>>>(pops_of<const __half>(s), ph, s.g, K, lt, 0);
-      else k_two_f16v2<<<grid, 256, 0, st>>>(pops_of<const __half>(s), ph, s.g, K, lt);
+      const dim3 grid((unsigned)(((long long)s.g.ny * r.tpr + 255) / 256), s.g.nz);
+      k_two_f16v2<<<grid, 256, 0, st>>>(pops_of<const __half>(s), ph, s.g, K, r.arg);
       return cudaGetLastError();
     }
   }
@@ -1686,12 +1633,9 @@ cudaError_t launch_step_out_of_place(const Lattice& src, const Lattice& dst, dou
       k_two<F64><<<sh.grid, sh.block, 0, st>>>(pops_of<const double>(src), pops_of<double>(dst), src.g, K);
       return cudaGetLastError();
     case FORM_F32: {
-      const int lt2 = vec_log_tpr(src.g, 2);
-      if (lt2 >= 0)
-        k_two_f32v<false><<<vec_grid(src.g, lt2, src.g.nz), 128, 0, st>>>(pops_of<const float>(src),
-                                                                           pops_of<float>(dst), src.g, K, lt2, 0);
-      else
-        k_two<F32><<<sh.grid, sh.block, 0, st>>>(pops_of<const float>(src), pops_of<float>(dst), src.g, K);
+      const VecRows r(src.g, 2, true);
+      launch_vec(k_two_f32v<false, false>, k_two_f32v<false, true>, src.g, r, src.g.nz, st, pops_of<const float>(src),
+                 pops_of<float>(dst), src.g, K, r.arg, 0);
       return cudaGetLastError();
     }
   }
@@ -1713,69 +1657,58 @@ template <class F>
 static cudaError_t aa_impl(const Lattice& a, int odd, const StepK& K, int variant, cudaStream_t st) {
   using S = typename F::S;
   Shape sh = cell_shape(a.g);
-  const int lt4 = F::id == FORM_F16 && (variant == 0 || variant == 4) ? vec_log_tpr(a.g, 4) : -1;
-  // FP32: two cells per thread where the box fits it (automatic or 2): on
-  // B200 the pair of AA steps measured 41.9 GLUPS against 39.8 with one cell
-  // per thread at 256^3 (40.5 against 38.9 at 1024^3), the Smagorinsky pair
-  // 40.6 against 34.1
-  const int lt2 = F::id == FORM_F32 && (variant == 0 || variant == 2) ? vec_log_tpr(a.g, 2) : -1;
-  // FP32 odd step (automatic): four cells per thread where the box fits it;
-  // the pair of AA steps measured 44.1 GLUPS at 256^3 and 44.2 at 512^3
-  // against 42.2 and 40.8 with two cells per thread on both steps, and with
-  // the Smagorinsky collision 43.9 against 40.9 at 256^3 (in FP16 eight cells
-  // gave the Smagorinsky odd step nothing: 76.0 against 76.2, issue-bound)
-  const int lt4f = F::id == FORM_F32 && variant == 0 && odd ? vec_log_tpr(a.g, 4) : -1;
-  if (lt4f >= 0) {
-    const dim3 grid = vec_grid(a.g, lt4f, a.g.nz);
-    if (K.les) k_aa_f32w<true><<<grid, 128, 0, st>>>(pops_of<float>(a), a.g, K, lt4f);
-    else k_aa_f32w<false><<<grid, 128, 0, st>>>(pops_of<float>(a), a.g, K, lt4f);
+  // FP32 (automatic or 2): two cells per thread; the pair of AA steps measured
+  // 41.9 GLUPS against 39.8 with one cell per thread at 256^3 on B200 (40.5
+  // against 38.9 at 1024^3), the Smagorinsky pair 40.6 against 34.1. The
+  // automatic odd step has four cells per thread where rows are whole chunks:
+  // 44.1 GLUPS for the pair at 256^3 and 44.2 at 512^3 against 42.2 and 40.8,
+  // with the Smagorinsky collision 43.9 against 40.9
+  const bool big = (long long)a.g.nx * a.g.ny * a.g.nz >= VEC_MIN_AA;
+  if (F::id == FORM_F32 && (variant == 2 || (variant == 0 && big))) {
+    const Pops<float> pf = pops_of<float>(a);
+    const VecRows r4(a.g, 4, false, true), r(a.g, 2, false);
+    if (odd && variant == 0 && r4.arg >= 0) {
+      if (K.les) launch_vec(k_aa_f32w<true, false>, k_aa_f32w<true, true>, a.g, r4, a.g.nz, st, pf, a.g, K, r4.arg);
+      else launch_vec(k_aa_f32w<false, false>, k_aa_f32w<false, true>, a.g, r4, a.g.nz, st, pf, a.g, K, r4.arg);
+    } else if (K.les) {
+      if (odd) launch_vec(k_aa_f32v<true, true, false>, k_aa_f32v<true, true, true>, a.g, r, a.g.nz, st, pf, a.g, K, r.arg);
+      else launch_vec(k_aa_f32v<false, true, false>, k_aa_f32v<false, true, true>, a.g, r, a.g.nz, st, pf, a.g, K, r.arg);
+    } else {
+      if (odd) launch_vec(k_aa_f32v<true, false, false>, k_aa_f32v<true, false, true>, a.g, r, a.g.nz, st, pf, a.g, K, r.arg);
+      else launch_vec(k_aa_f32v<false, false, false>, k_aa_f32v<false, false, true>, a.g, r, a.g.nz, st, pf, a.g, K, r.arg);
+    }
     return cudaGetLastError();
   }
-  if (lt2 >= 0) {
-    const dim3 grid = vec_grid(a.g, lt2, a.g.nz);
-    Pops<float> pf = pops_of<float>(a);
+  // FP16 (automatic or 4): four cells per thread. The automatic BGK odd step has
+  // eight where rows are whole chunks: on B200 the pair of AA steps measured
+  // 84.3 GLUPS at 256^3 and 86.0 at 512^3 against 80.0 and 81.6 with four cells
+  // per thread on both steps; eight cells on the even step as well measured the
+  // same (84.1, 86.1), so the even step stays on k_aa_f16v, and eight cells gave
+  // the Smagorinsky odd step nothing (76.0 against 76.2, issue-bound). Rows of no
+  // power of two: 384 x 256 x 256 79.8 against 56.4 on one cell per thread
+  if (F::id == FORM_F16 && (variant == 4 || (variant == 0 && big))) {
+    const Pops<__half> ph = pops_of<__half>(a);
+    const VecRows r8(a.g, 8, false, true), r(a.g, 4, false);
     if (K.les) {
-      if (odd) k_aa_f32v<true, true><<<grid, 128, 0, st>>>(pf, a.g, K, lt2);
-      else k_aa_f32v<false, true><<<grid, 128, 0, st>>>(pf, a.g, K, lt2);
+      if (odd) launch_vec(k_aa_f16v<true, true, false>, k_aa_f16v<true, true, true>, a.g, r, a.g.nz, st, ph, a.g, K, r.arg);
+      else launch_vec(k_aa_f16v<false, true, false>, k_aa_f16v<false, true, true>, a.g, r, a.g.nz, st, ph, a.g, K, r.arg);
+    } else if (odd && variant == 0 && r8.arg >= 0) {
+      launch_vec(k_aa_f16w<true, false>, k_aa_f16w<true, true>, a.g, r8, a.g.nz, st, ph, a.g, K, r8.arg);
     } else {
-      if (odd) k_aa_f32v<true, false><<<grid, 128, 0, st>>>(pf, a.g, K, lt2);
-      else k_aa_f32v<false, false><<<grid, 128, 0, st>>>(pf, a.g, K, lt2);
+      if (odd) launch_vec(k_aa_f16v<true, false, false>, k_aa_f16v<true, false, true>, a.g, r, a.g.nz, st, ph, a.g, K, r.arg);
+      else launch_vec(k_aa_f16v<false, false, false>, k_aa_f16v<false, false, true>, a.g, r, a.g.nz, st, ph, a.g, K, r.arg);
     }
     return cudaGetLastError();
   }
   if (K.les) {
-    if (lt4 >= 0) {
-      const dim3 grid = vec_grid(a.g, lt4, a.g.nz);
-      if (odd) k_aa_f16v<true, true><<<grid, 128, 0, st>>>(pops_of<__half>(a), a.g, K, lt4);
-      else k_aa_f16v<false, true><<<grid, 128, 0, st>>>(pops_of<__half>(a), a.g, K, lt4);
-    } else if (odd) {
-      k_aa<F, true, true><<<sh.grid, sh.block, 0, st>>>(pops_of<S>(a), a.g, K);
-    } else {
-      k_aa<F, false, true><<<sh.grid, sh.block, 0, st>>>(pops_of<S>(a), a.g, K);
-    }
+    if (odd) k_aa<F, true, true><<<sh.grid, sh.block, 0, st>>>(pops_of<S>(a), a.g, K);
+    else k_aa<F, false, true><<<sh.grid, sh.block, 0, st>>>(pops_of<S>(a), a.g, K);
     return cudaGetLastError();
   }
   if (variant == 8) {
     bool launched = false;
     cudaError_t e = launch_rows(a, a, odd ? ROW_AA_ODD : ROW_AA_EVEN, K, st, &launched);
     if (e != cudaSuccess || launched) return e;
-  }
-  // FP16 odd step (automatic): eight cells per thread where the box fits it.
-  // On B200 the pair of AA steps measured 84.3 GLUPS at 256^3 and 86.0 at
-  // 512^3 against 80.0 and 81.6 with four cells per thread on both steps;
-  // eight cells on the even step as well measured the same (84.1, 86.1), so
-  // the even step stays on k_aa_f16v (96 registers, 5 blocks/SM)
-  const int lt8 = F::id == FORM_F16 && variant == 0 && odd ? vec_log_tpr(a.g, 8) : -1;
-  if (lt8 >= 0) {
-    k_aa_f16w<true><<<vec_grid(a.g, lt8, a.g.nz), 128, 0, st>>>(pops_of<__half>(a), a.g, K, lt8);
-    return cudaGetLastError();
-  }
-  // FP16: four cells per thread where the box fits it (automatic or 4)
-  if (lt4 >= 0) {
-    const dim3 grid = vec_grid(a.g, lt4, a.g.nz);
-    if (odd) k_aa_f16v<true, false><<<grid, 128, 0, st>>>(pops_of<__half>(a), a.g, K, lt4);
-    else k_aa_f16v<false, false><<<grid, 128, 0, st>>>(pops_of<__half>(a), a.g, K, lt4);
-    return cudaGetLastError();
   }
   if (odd && F::id == FORM_F16)
     k_aa_f16_odd<<<sh.grid, sh.block, 0, st>>>(pops_of<__half>(a), a.g, K);
@@ -1978,22 +1911,21 @@ static cudaError_t slab_impl(const Lattice& s, const Lattice& d, const StepK& K,
   else k_slab<F, false, true><<<ge, sh.block, 0, st>>>(ps, pd, s.g, K, h);
   if (s.g.nz > 2) {
     // FP16 / FP32: the interior planes on the four- / two-cells-per-thread
-    // kernel where the rows fit it (planes 1 .. nz-2 pull only inside the
-    // slab, so its z wrap never applies)
-    const int lt = F::id == FORM_F16 ? vec_log_tpr(s.g, 4) : -1;
-    const int lt2 = F::id == FORM_F32 ? vec_log_tpr(s.g, 2) : -1;
-    if (lt2 >= 0) {
+    // kernel (planes 1 .. nz-2 pull only inside the slab, so its z wrap never
+    // applies)
+    const int ni = s.g.nz - 2;
+    if (F::id == FORM_F32) {
       Pops<float> pf = pops_of<float>(d);
       pf.p[Q - 1] = (float*)s.p[Q - 1];
-      const dim3 gv = vec_grid(s.g, lt2, s.g.nz - 2);
-      if (K.les) k_two_f32v<true><<<gv, 128, 0, st_in>>>(pops_of<const float>(s), pf, s.g, K, lt2, 1);
-      else k_two_f32v<false><<<gv, 128, 0, st_in>>>(pops_of<const float>(s), pf, s.g, K, lt2, 1);
-    } else if (lt >= 0) {
+      const VecRows r(s.g, 2, true);
+      if (K.les) launch_vec(k_two_f32v<true, false>, k_two_f32v<true, true>, s.g, r, ni, st_in, pops_of<const float>(s), pf, s.g, K, r.arg, 1);
+      else launch_vec(k_two_f32v<false, false>, k_two_f32v<false, true>, s.g, r, ni, st_in, pops_of<const float>(s), pf, s.g, K, r.arg, 1);
+    } else if (F::id == FORM_F16) {
       Pops<__half> ph = pops_of<__half>(d);
       ph.p[Q - 1] = (__half*)s.p[Q - 1];
-      const dim3 gv = vec_grid(s.g, lt, s.g.nz - 2);
-      if (K.les) k_two_f16v<true><<<gv, 128, 0, st_in>>>(pops_of<const __half>(s), ph, s.g, K, lt, 1);
-      else k_two_f16v<false><<<gv, 128, 0, st_in>>>(pops_of<const __half>(s), ph, s.g, K, lt, 1);
+      const VecRows r(s.g, 4, true);
+      if (K.les) launch_vec(k_two_f16v<true, false>, k_two_f16v<true, true>, s.g, r, ni, st_in, pops_of<const __half>(s), ph, s.g, K, r.arg, 1);
+      else launch_vec(k_two_f16v<false, false>, k_two_f16v<false, true>, s.g, r, ni, st_in, pops_of<const __half>(s), ph, s.g, K, r.arg, 1);
     } else {
       const dim3 gi(sh.grid.x, sh.grid.y, s.g.nz - 2);
       if (K.les) k_slab<F, true, false><<<gi, sh.block, 0, st_in>>>(ps, pd, s.g, K, h);

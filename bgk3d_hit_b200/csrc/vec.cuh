@@ -52,27 +52,109 @@ __device__ __forceinline__ void collide4_f16(uint2 (&Y)[Q], const StepK& K) {
   }
 }
 
-// Lanes that exchange x-neighbours in the several-cells-per-thread kernels:
-// a row of nx cells is tpr = nx/V consecutive threads (V cells per thread).
-// Rows shorter than a warp wrap inside it; rows of one or more warps wrap
-// through global memory at the warp's first / last lane (edge_prev /
-// edge_next).
+// Place of a thread of a several-cells-per-thread kernel (V cells of a row per
+// thread, 128-thread blocks over the ny*tpr threads of a plane).
+// FLAT = false: nx/V = tpr is a power of two (arg = its logarithm) and ny*tpr a
+// multiple of 32, so warps and rows are aligned with each other. FLAT = true:
+// any nx, arg = tpr; row boundaries fall anywhere in a warp, the last chunk with
+// cells may hold only `cells` < V of them, and chunks behind it (pad, where the
+// launch asks for padded rows) work on the row's padding. Nothing in the
+// padding ever reaches a cell.
+template <int V, bool FLAT> struct VecPlace {
+  int tpr, j, pos;
+  int i0, i_prev, i_next;  // first cell, and the (periodic) elements before and behind the chunk
+  int cells;               // cells of the row's last chunk
+  bool valid;              // false: past the plane's last thread; j is clamped
+  bool end;                // the row's last chunk with cells, or behind it
+  __device__ VecPlace(const Geo& g, int arg) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (FLAT) {
+      tpr = arg;
+      j = (int)((unsigned)t / (unsigned)tpr);
+      pos = t - j * tpr;
+      const int e = (g.nx - 1) / V;
+      cells = g.nx - V * e;
+      end = pos >= e;
+    } else {
+      tpr = 1 << arg;
+      j = t >> arg;
+      pos = t & (tpr - 1);
+      cells = V;
+      end = pos == tpr - 1;
+    }
+    valid = j < g.ny;
+    if (!valid) j = FLAT ? g.ny - 1 : 0;
+    i0 = pos * V;
+    i_prev = pos == 0 ? g.nx - 1 : i0 - 1;
+    i_next = end ? 0 : i0 + V;
+  }
+  __device__ bool last() const { return FLAT && end && cells < V; }
+};
+
+// Lanes that exchange x-neighbours in the several-cells-per-thread kernels.
+// Aligned rows shorter than a warp wrap inside it; rows of one or more warps
+// wrap through global memory at the warp's first / last lane (edge_prev /
+// edge_next). FLAT rows: the lanes at a row's ends are edges too.
 struct XLanes {
   int src_prev, src_next;
   bool edge_prev, edge_next;
-  __device__ XLanes(int tpr, int pos, int lane) {
+  template <int V, bool FLAT> __device__ XLanes(const VecPlace<V, FLAT>& at, int lane) {
     edge_prev = edge_next = false;
-    if (tpr >= 32) {
+    if (FLAT || at.tpr >= 32) {
       src_prev = (lane + 31) & 31;
       src_next = (lane + 1) & 31;
-      edge_prev = lane == 0;
-      edge_next = lane == 31;
+      edge_prev = lane == 0 || (FLAT && at.pos == 0);
+      edge_next = lane == 31 || (FLAT && at.end);
     } else {
-      src_prev = pos == 0 ? lane + tpr - 1 : lane - 1;
-      src_next = pos == tpr - 1 ? lane - tpr + 1 : lane + 1;
+      src_prev = at.pos == 0 ? lane + at.tpr - 1 : lane - 1;
+      src_next = at.pos == at.tpr - 1 ? lane - at.tpr + 1 : lane + 1;
     }
   }
 };
+
+// Neighbouring warps of the block that an AA odd step's warp-edge lanes pass
+// their crossing values to: prev_in / next_in where the row goes on in warp
+// wprev / wnext of the same block.
+struct EdgeWarps {
+  bool any, prev_in, next_in;
+  int wprev, wnext;
+  template <int V, bool FLAT> __device__ explicit EdgeWarps(const VecPlace<V, FLAT>& at) {
+    const int w = threadIdx.x >> 5;
+    any = FLAT || at.tpr >= 32;
+    prev_in = next_in = false;
+    wprev = w - 1;
+    wnext = w + 1;
+    if (FLAT) {
+      prev_in = w > 0 && at.pos != 0;
+      next_in = w < 3 && !at.end;
+    } else if (any) {
+      const int nw = at.tpr >> 5, r = at.pos >> 5;  // warps per row, this warp's place in its row
+      if (nw <= 4) {  // the whole row in this block
+        prev_in = next_in = true;
+        wprev = w - r + (r + nw - 1) % nw;
+        wnext = w - r + (r + 1) % nw;
+      } else {
+        prev_in = w > 0;
+        next_in = w < 3;
+      }
+    }
+  }
+};
+
+// In a row's last chunk of `cells` cells, the element behind the last cell is
+// the row's first one, which the lane loaded into E (pulls with cx < 0).
+__device__ __forceinline__ void wrap_last(uint2 (&Y)[Q], const unsigned short (&E)[Q], int cells) {
+#pragma unroll
+  for (int q = 9; q < 14; ++q) {
+    if (cells == 1) Y[q].x = __byte_perm(Y[q].x, E[q], 0x5410);
+    else if (cells == 2) Y[q].y = __byte_perm(Y[q].y, E[q], 0x3254);
+    else Y[q].y = __byte_perm(Y[q].y, E[q], 0x5410);
+  }
+}
+__device__ __forceinline__ void wrap_last(float2 (&Y)[Q], const float (&E)[Q], int) {
+#pragma unroll
+  for (int q = 9; q < 14; ++q) Y[q].y = E[q];
+}
 
 // Second half of the x-shifted row loads of the four-cells-per-thread FP16
 // kernels. Y[q] holds the aligned chunk of elements i0..i0+3 of population
@@ -120,16 +202,38 @@ __device__ __forceinline__ void shift_rows_f32(float2 (&Y)[Q], const float (&E)[
   }
 }
 
-// log2(nx/V) when a V-cells-per-thread kernel applies (nx/V a power of two,
-// whole warps per plane), else -1.
-inline int vec_log_tpr(const Geo& g, int V) {
-  if (g.nx % V) return -1;
-  const int tpr = g.nx / V;
-  if (tpr & (tpr - 1)) return -1;
-  if (((long long)g.ny * tpr) % 32) return -1;
-  int l = 0;
-  while ((1 << l) < tpr) ++l;
-  return l;
-}
+// Rows of a V-cells-per-thread kernel: aligned (arg = log2(nx/V)) where nx/V is
+// a power of two and a plane holds whole warps, else flat (arg = chunks of a
+// row). padded: up to a 32-byte sector (8-byte chunks), for kernels that write
+// rows they have not read: a partly written sector costs memory a read (FP16
+// two-lattice step at 180^3:
+// 74.3 GLUPS against 58.5 with rows cut at their last chunk, and 67 with zeros
+// stored by lanes of their own; the AA step has read its rows and gains nothing). whole: only rows of whole chunks (the
+// 16-byte kernels); arg < 0: not for them.
+struct VecRows {
+  bool flat;
+  int arg, tpr;
+  VecRows(const Geo& g, int V, bool padded, bool whole = false)
+      : flat(true), arg(padded ? (g.nx + 4 * V - 1) / (4 * V) * 4 : (g.nx + V - 1) / V), tpr(arg) {
+    if (whole && g.nx % V) {
+      arg = -1;
+      return;
+    }
+    const int t = g.nx / V;
+    if (g.nx % V || (t & (t - 1)) || ((long long)g.ny * t) % 32) return;
+    flat = false;
+    tpr = t;
+    arg = 0;
+    while ((1 << arg) < tpr) ++arg;
+  }
+};
+
+
+// From how many cells the automatic choice takes the several-cells-per-thread
+// kernels: below, their fewer and longer threads leave the chip idle and one
+// cell per thread is faster. Measured us per step, one cell / several: AA FP16
+// 32^3 4.1 / 5.1, 48^3 6.2 / 7.2, 210,000 cells 7.8 / 8.6, 64^3 7.7 / 7.2; FP32
+// two-lattice 33^3 4.1 / 5.1, 48^3 6.2 / 6.2, 66^3 10.3 / 8.2.
+constexpr long long VEC_MIN_TWO = 1LL << 17, VEC_MIN_AA = 1LL << 18;
 
 }  // namespace bgk
