@@ -20,7 +20,7 @@ ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 INCLUDE = os.path.join(ROOT, "include")
 OUT = os.path.join(HERE, "libbgk3d.so")
-SOURCES = ["kernels.cu", "rows.cu", "adjoint.cu", "bgk_abi.cu", "noalloc.cu"]
+SOURCES = ["kernels.cu", "fused.cu", "rows.cu", "adjoint.cu", "bgk_abi.cu", "noalloc.cu"]
 HEADERS = ["lattice.cuh", "kernels.h", "reduce.cuh", "vec.cuh"]
 ARCH = "-gencode=arch=compute_100a,code=sm_100a"
 

@@ -9,6 +9,7 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "bgk3d.h"
@@ -55,6 +56,7 @@ constexpr size_t POP_STAGE_BYTES = 64u << 20;
 struct bgk_ctx {
   bgk_params p;
   int form = 0, scheme = 0;
+  int fused = 0;  // bgk_run takes two steps per launch (launch_two_steps)
   cudaStream_t st = nullptr;
   cudaEvent_t mark = nullptr;  // bgk_record_event / bgk_wait_event
   // z-slab: second stream for the interior planes and its fork / join events
@@ -666,12 +668,18 @@ int bgk_create(const bgk_params* p, bgk_ctx** out) {
   if (rc) return fail(rc);
   for (int q = 0; q < Q; ++q) c->A.p[q] = (char*)c->memA + q * pop_bytes;
   if (c->scheme == BGK_TWO_LATTICE) {
-    // b01..b18; b19 is never used (pop 19 is updated in place,
-    // SRC/col_MC.F90:351), so it is not allocated
-    rc = dev_alloc(c, &c->memB, (Q - 1) * pop_bytes, "lattice b");
-    if (rc) return fail(rc);
+    // b01..b18, and b19 where two steps run as one: a single step updates pop 19
+    // in place (SRC/col_MC.F90:351) and needs no second one. Without the memory
+    // for it the box runs single steps
+    c->fused = p->kernel == 0 && !c->slab && p->mode == BGK_CORRECTED &&
+               two_steps_pay(c->g, c->form, p->les_cs > 0.0);
+    if (c->fused && dev_alloc(c, &c->memB, Q * pop_bytes, "lattice b")) c->fused = 0;
+    if (!c->fused) {
+      rc = dev_alloc(c, &c->memB, (Q - 1) * pop_bytes, "lattice b");
+      if (rc) return fail(rc);
+    }
     for (int q = 0; q < Q - 1; ++q) c->B.p[q] = (char*)c->memB + q * pop_bytes;
-    c->B.p[Q - 1] = c->A.p[Q - 1];
+    c->B.p[Q - 1] = c->fused ? (char*)c->memB + (Q - 1) * pop_bytes : c->A.p[Q - 1];
   }
   rc = dev_alloc(c, (void**)&c->partials, (size_t)DIAG_BLOCKS * ND * 2 * sizeof(double), "diagnostic partials");
   if (rc) return fail(rc);
@@ -961,7 +969,17 @@ int bgk_run(bgk_ctx* c, int nsteps) {
     set_err("z-slab: one step per call, with the slabs synchronised between steps");
     return BGK_ERR_INVALID;
   }
-  for (int s = 0; s < nsteps; ++s) {
+  int s = 0;
+  if (c && c->fused && c->initialized && nsteps >= 2) {
+    CK(cudaSetDevice(c->p.device));
+    for (; s + 2 <= nsteps; s += 2) {
+      CK(launch_two_steps(c->A, c->B, c->omega, c->scale, c->p.les_cs, c->st));
+      std::swap(c->A, c->B);  // all 19 populations are in b
+      c->launches++;
+      c->step += 2;
+    }
+  }
+  for (; s < nsteps; ++s) {
     int rc = bgk_boundaries(c, (int)(c ? c->step + 1 : 0));
     if (rc) return rc;
     rc = bgk_col_mc(c, (int)(c->step + 1));

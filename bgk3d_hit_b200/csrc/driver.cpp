@@ -16,6 +16,7 @@
 //   lx*ly*lz*(itfin - itstart)/(loop seconds * 1e9).
 // Exit status 0 on success, 1 on a library error (its message on stderr).
 #include <cctype>
+#include <algorithm>
 #include <chrono>
 #include <cmath>
 #include <cstdio>
@@ -167,9 +168,12 @@ int main(int argc, char** argv) {
   if (ivtim > 0 && slices(0)) return fail("bgk_vtk");
   if (bgk_synchronize(ctx)) return fail("bgk_synchronize");
   const auto t0 = std::chrono::steady_clock::now();
-  for (int itime = itstart; itime <= itfin; ++itime) {
-    if (bgk_boundaries(ctx, itime)) return fail("bgk_boundaries");
-    if (bgk_col_mc(ctx, itime)) return fail("bgk_col_mc");
+  // boundaries + col_MC up to the next step that is looked at, in one call
+  for (int itime = itstart - 1; itime < itfin;) {
+    int n = std::min(itfin - itime, p.icheck - itime % p.icheck);
+    if (itsave > 0) n = std::min(n, itsave - itime % itsave);
+    if (bgk_run(ctx, n)) return fail("bgk_run");
+    itime += n;
     bgk_diag d;
     const int rc = bgk_diagnostic(ctx, itime, &d);
     if (rc < 0) return fail("bgk_diagnostic");

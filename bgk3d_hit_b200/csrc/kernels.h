@@ -52,6 +52,14 @@ cudaError_t launch_two_lattice(const Lattice& src, const Lattice& dst, double om
 // FP64 and FP32 forms (used by the adjoint's recomputation).
 cudaError_t launch_step_out_of_place(const Lattice& src, const Lattice& dst, double omega, cudaStream_t st);
 
+// Two consecutive steps src -> dst in one pass, all 19 populations written to dst
+// (dst.p[18] must not be src.p[18]); populations 0..17 of src follow each other
+// every g.qs elements. FP64 and FP32 (BGK) boxes for which two_steps_pay. src.err
+// is set when a copy did not land.
+bool two_steps_pay(const Geo& g, int form, bool les);
+cudaError_t launch_two_steps(const Lattice& src, const Lattice& dst, double omega, double scale, double les_cs,
+                             cudaStream_t st);
+
 // ------------------------------------------------------------- adjoint
 // Terminal adjoint and loss: lam = dL/df for L = 0.5 mean|u(f) - u_tgt|^2;
 // the loss is accumulated into acc (one compensated pair per block).

@@ -309,6 +309,8 @@ def run_loop(box: BGK3D, itfin: int, out_dir: str | None = None, itstart: int = 
     """Replays the time loop of SRC/bgk3d_HIT.F90:127-146 (boundaries, col_MC,
     diagnostic) and returns the diagnostic records; with out_dir, writes
     diagno.dat and dissipation.dat in the reference's formats (i8, e14.6).
+    The steps between two that are looked at (diagnostic every icheck, itsave)
+    go to the library in one call.
     With ivtim, also the three mid-box VTK slices at itime 0 and on every
     diagnostic step that is a multiple of ivtim (SRC/bgk3d_HIT.F90:118-120,
     SRC/diagnostic.F90:52-58); with itsave, a checkpoint every itsave steps."""
@@ -324,9 +326,14 @@ def run_loop(box: BGK3D, itfin: int, out_dir: str | None = None, itstart: int = 
         os.makedirs(out_dir, exist_ok=True)
         if ivtim:
             slices(0)
-    for itime in range(itstart, itfin + 1):
-        box.boundaries(itime)
-        box.col_MC(itime)
+    every = [box.params.icheck] + ([itsave] if out_dir and itsave else [])
+    itime = itstart - 1
+    while itime < itfin:
+        n = min([itfin - itime] + [k - itime % k for k in every])
+        if box.params.proc_z > 1:  # a z-slab takes one step per call
+            n = 1
+        box.run(n)
+        itime += n
         d = box.diagnostic(itime)
         if d is not None:
             recs.append(d)

@@ -172,7 +172,12 @@ int bgk_boundaries(bgk_ctx* ctx, int itime);
    layout flip (AA). Asynchronous. */
 int bgk_col_mc(bgk_ctx* ctx, int itime);
 
-/* Runs nsteps consecutive bgk_boundaries + bgk_col_mc steps. Asynchronous. */
+/* Runs nsteps consecutive bgk_boundaries + bgk_col_mc steps. Asynchronous. With
+   the automatic kernel, larger two-lattice boxes in corrected mode (FP64, and FP32
+   without the LES collision) take two steps per launch and one pass over the
+   populations, with the results of single steps; bgk_create allocates a second
+   population 19 for them (38 arrays instead of 37) and leaves it at single steps
+   where that does not fit the device. */
 int bgk_run(bgk_ctx* ctx, int nsteps);
 
 /* = diagnostic(itime, icheck, ...) (SRC/diagnostic.F90:25-75): when
