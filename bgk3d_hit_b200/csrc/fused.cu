@@ -137,6 +137,11 @@ __global__ void __launch_bounds__(Two2<typename F::S, TY>::THREADS, 1)
   };
   auto next = [&](int p) { return p == g.nz - 1 ? 0 : p + 1; };
 
+  // a step after this one may be scheduled now; nothing of the step before is read
+  // or overwritten before it is done (step_begin of the single steps)
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+
   if (tid == T::WORK) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&sm.bar[0])) : "memory");
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&sm.bar[1])) : "memory");
@@ -351,8 +356,17 @@ cudaError_t launch(const Lattice& s, const Lattice& d, const StepK& K, cudaStrea
     return cudaErrorInvalidValue;
   const int lz = best_walk(g, TY, SMS).lz;
   const dim3 grid((g.nx + TX - 1) / TX, (g.ny + TY - 1) / TY, (g.nz + lz - 1) / lz);
-  kern<<<grid, T::THREADS, bytes, st>>>(m, pops<const S>(s), pops<S>(d), g, K, lz, s.err);
-  return cudaGetLastError();
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(T::THREADS);
+  cfg.dynamicSmemBytes = bytes;
+  cfg.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, m, pops<const S>(s), pops<S>(d), g, K, lz, s.err);
 }
 
 }  // namespace

@@ -35,6 +35,17 @@ __device__ __forceinline__ double ldg(const double* p) { return __ldg(p); }
 __device__ __forceinline__ float ldg(const float* p) { return __ldg(p); }
 __device__ __forceinline__ __half ldg(const __half* p) { return __ldg(p); }
 
+// Consecutive steps overlap their launches: a step's blocks are scheduled while the
+// last blocks of the step before still run (launch_step asks for it), and wait here
+// until all of that step's stores can be seen. First statement of every kernel
+// that launch_step launches. us per step without / with it on B200: FP64 32^3 4.1 /
+// 3.2, 64^3 10.7 / 9.0, 128^3 98.6 / 95.9; FP16 32^3 4.1 / 2.2, 64^3 6.2 / 4.9, 128^3
+// 28.7 / 26.0.
+__device__ __forceinline__ void step_begin() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // Moments of 19 local deviations in the reference's order
 // (SRC/diagno.F90:96-104, identical to SRC/col_MC.F90:133-141).
 template <class V>
@@ -62,6 +73,22 @@ static Shape cell_shape(const Geo& g) {
   return s;
 }
 
+// Launches a step kernel so that it may be scheduled beside the end of the kernel
+// before it in the stream (see step_begin).
+template <class... P, class... A>
+static cudaError_t launch_step(void (*kern)(P...), dim3 grid, dim3 block, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
+
 static int grid_1d(long long n, int threads, int cap) {
   long long b = (n + threads - 1) / threads;
   return (int)(b < cap ? (b < 1 ? 1 : b) : cap);
@@ -70,6 +97,7 @@ static int grid_1d(long long n, int threads, int cap) {
 // ------------------------------------------------------------- two lattice
 template <class F, bool LES = false>
 __global__ void __launch_bounds__(256) k_two(Pops<const typename F::S> src, Pops<typename F::S> dst, Geo g, StepK K) {
+  step_begin();
   using S = typename F::S;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
@@ -115,6 +143,7 @@ __global__ void __launch_bounds__(256) k_two(Pops<const typename F::S> src, Pops
 template <bool LES, bool FLAT>
 __global__ void __launch_bounds__(128, 5) k_two_f16v(Pops<const __half> src, Pops<__half> dst, Geo g, StepK K,
                                                   int rows, int k0) {
+  step_begin();
   const VecPlace<4, FLAT> at(g, rows);
   const int k = blockIdx.y + k0;  // planes k0 .. k0 + gridDim.y - 1
   if (!at.valid) return;  // whole warps unless FLAT; no lane needs a value of theirs
@@ -150,6 +179,7 @@ __global__ void __launch_bounds__(128, 5) k_two_f16v(Pops<const __half> src, Pop
 template <bool LES, bool FLAT>
 __global__ void __launch_bounds__(128, 5) k_two_f32v(Pops<const float> src, Pops<float> dst, Geo g, StepK K,
                                                   int rows, int k0) {
+  step_begin();
   const VecPlace<2, FLAT> at(g, rows);
   const int k = blockIdx.y + k0;  // planes k0 .. k0 + gridDim.y - 1
   if (!at.valid) return;  // whole warps unless FLAT; no lane needs a value of theirs
@@ -194,6 +224,7 @@ __global__ void __launch_bounds__(128, 5) k_two_f32v(Pops<const float> src, Pops
 // nx/2 threads per row); otherwise as k_two_f16v.
 __global__ void __launch_bounds__(256, 4) k_two_f16v2(Pops<const __half> src, Pops<__half> dst, Geo g, StepK K,
                                                    int log_tpr) {
+  step_begin();
   const int tpr = 1 << log_tpr;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = t >> log_tpr, pos = t & (tpr - 1);
@@ -302,6 +333,7 @@ __device__ __forceinline__ void aa_cell(Pops<typename F::S>& a, const Geo& g, co
 
 template <class F, bool ODD, bool LES = false>
 __global__ void __launch_bounds__(256) k_aa(Pops<typename F::S> a, Geo g, StepK K) {
+  step_begin();
   aa_cell<F, ODD, LES>(a, g, K);
 }
 
@@ -309,6 +341,7 @@ __global__ void __launch_bounds__(256) k_aa(Pops<typename F::S> a, Geo g, StepK 
 // blocks per SM) it measured 53.7 against 50.4 GLUPS uncapped for that step at
 // 256^3 on B200, a few spilled bytes included.
 __global__ void __launch_bounds__(256, 5) k_aa_f16_odd(Pops<__half> a, Geo g, StepK K) {
+  step_begin();
   aa_cell<F16, true, false>(a, g, K);
 }
 
@@ -388,6 +421,7 @@ __device__ __forceinline__ void shift_out(uint2 Y, int cx, __half* p, const VecP
 
 template <bool ODD, bool LES, bool FLAT>
 __global__ void __launch_bounds__(128, 5) k_aa_f16v(Pops<__half> a, Geo g, StepK K, int rows) {
+  step_begin();
   const VecPlace<4, FLAT> at(g, rows);
   const int k = blockIdx.y;
   const bool valid = at.valid;  // whole warps unless FLAT
@@ -536,6 +570,7 @@ __device__ __forceinline__ void shift_out8(uint4 Y, int cx, __half* p, const Vec
 
 template <bool ODD, bool FLAT>
 __global__ void __launch_bounds__(128, 4) k_aa_f16w(Pops<__half> a, Geo g, StepK K, int rows) {
+  step_begin();
   const VecPlace<8, FLAT> at(g, rows);
   const int k = blockIdx.y;
   const bool valid = at.valid;  // whole warps unless FLAT
@@ -651,6 +686,7 @@ __device__ __forceinline__ void shift_out_f32(float2 Y, int cx, float* p, const 
 // for the Smagorinsky even step), no spills.
 template <bool ODD, bool LES, bool FLAT>
 __global__ void __launch_bounds__(128, 5) k_aa_f32v(Pops<float> a, Geo g, StepK K, int rows) {
+  step_begin();
   const VecPlace<2, FLAT> at(g, rows);
   const int k = blockIdx.y;
   const bool valid = at.valid;  // whole warps unless FLAT
@@ -773,6 +809,7 @@ __device__ __forceinline__ void shift_out4_f32(float4 Y, int cx, float* p, const
 
 template <bool LES, bool FLAT>
 __global__ void __launch_bounds__(128, 4) k_aa_f32w(Pops<float> a, Geo g, StepK K, int rows) {
+  step_begin();
   const VecPlace<4, FLAT> at(g, rows);
   const int k = blockIdx.y;
   const bool valid = at.valid;  // whole warps unless FLAT
@@ -1563,11 +1600,19 @@ StepK make_stepk(int form, double omega, double scale, double les_cs) {
 
 // Launches a several-cells-per-thread kernel (its aligned and its flat
 // instantiation) in 128-thread blocks over the threads of `planes` planes.
-template <class KA, class KF, class... Args>
-static void launch_vec(KA aligned, KF flat, const Geo& g, const VecRows& r, int planes, cudaStream_t st, Args... args) {
+template <class... P, class... A>
+static cudaError_t launch_vec(void (*aligned)(P...), void (*flat)(P...), const Geo& g, const VecRows& r, int planes,
+                              cudaStream_t st, A... args) {
   const dim3 grid((unsigned)(((long long)g.ny * r.tpr + 127) / 128), (unsigned)planes);
-  if (r.flat) flat<<<grid, 128, 0, st>>>(args...);
-  else aligned<<<grid, 128, 0, st>>>(args...);
+  return launch_step(r.flat ? flat : aligned, grid, dim3(128), st, args...);
+}
+// The same as an ordinary launch, for a stream that is ordered by events.
+template <class... P, class... A>
+static void launch_vec_plain(void (*aligned)(P...), void (*flat)(P...), const Geo& g, const VecRows& r, int planes,
+                             cudaStream_t st, A... args) {
+  const dim3 grid((unsigned)(((long long)g.ny * r.tpr + 127) / 128), (unsigned)planes);
+  if (r.flat) flat<<<grid, 128, 0, st>>>(P(args)...);
+  else aligned<<<grid, 128, 0, st>>>(P(args)...);
 }
 
 template <class F>
@@ -1586,9 +1631,8 @@ static cudaError_t two_impl(const Lattice& s, const Lattice& d, const StepK& K, 
     Pops<float> pf = pops_of<float>(d);
     pf.p[Q - 1] = (float*)s.p[Q - 1];
     const VecRows r(s.g, 2, true);
-    if (K.les) launch_vec(k_two_f32v<true, false>, k_two_f32v<true, true>, s.g, r, s.g.nz, st, pops_of<const float>(s), pf, s.g, K, r.arg, 0);
-    else launch_vec(k_two_f32v<false, false>, k_two_f32v<false, true>, s.g, r, s.g.nz, st, pops_of<const float>(s), pf, s.g, K, r.arg, 0);
-    return cudaGetLastError();
+    if (K.les) return launch_vec(k_two_f32v<true, false>, k_two_f32v<true, true>, s.g, r, s.g.nz, st, pops_of<const float>(s), pf, s.g, K, r.arg, 0);
+    return launch_vec(k_two_f32v<false, false>, k_two_f32v<false, true>, s.g, r, s.g.nz, st, pops_of<const float>(s), pf, s.g, K, r.arg, 0);
   }
   // FP16: four cells per thread (automatic or 4; the Smagorinsky step too), the
   // fastest measured on B200 at 256^3 (76.6 GLUPS against 64.0 with one, 62.7
@@ -1598,13 +1642,11 @@ static cudaError_t two_impl(const Lattice& s, const Lattice& d, const StepK& K, 
     Pops<__half> ph = pops_of<__half>(d);
     ph.p[Q - 1] = (__half*)s.p[Q - 1];
     const VecRows r(s.g, 4, true);
-    if (K.les) launch_vec(k_two_f16v<true, false>, k_two_f16v<true, true>, s.g, r, s.g.nz, st, pops_of<const __half>(s), ph, s.g, K, r.arg, 0);
-    else launch_vec(k_two_f16v<false, false>, k_two_f16v<false, true>, s.g, r, s.g.nz, st, pops_of<const __half>(s), ph, s.g, K, r.arg, 0);
-    return cudaGetLastError();
+    if (K.les) return launch_vec(k_two_f16v<true, false>, k_two_f16v<true, true>, s.g, r, s.g.nz, st, pops_of<const __half>(s), ph, s.g, K, r.arg, 0);
+    return launch_vec(k_two_f16v<false, false>, k_two_f16v<false, true>, s.g, r, s.g.nz, st, pops_of<const __half>(s), ph, s.g, K, r.arg, 0);
   }
   if (K.les) {  // the other choices run the Smagorinsky collision on one cell per thread
-    k_two<F, true><<<sh.grid, sh.block, 0, st>>>(ps, pd, s.g, K);
-    return cudaGetLastError();
+    return launch_step(k_two<F, true>, sh.grid, sh.block, st, ps, pd, s.g, K);
   }
   if (variant == 8) {
     bool launched = false;
@@ -1617,12 +1659,10 @@ static cudaError_t two_impl(const Lattice& s, const Lattice& d, const StepK& K, 
       Pops<__half> ph = pops_of<__half>(d);
       ph.p[Q - 1] = (__half*)s.p[Q - 1];
       const dim3 grid((unsigned)(((long long)s.g.ny * r.tpr + 255) / 256), s.g.nz);
-      k_two_f16v2<<<grid, 256, 0, st>>>(pops_of<const __half>(s), ph, s.g, K, r.arg);
-      return cudaGetLastError();
+      return launch_step(k_two_f16v2, grid, 256, st, pops_of<const __half>(s), ph, s.g, K, r.arg);
     }
   }
-  k_two<F><<<sh.grid, sh.block, 0, st>>>(ps, pd, s.g, K);
-  return cudaGetLastError();
+  return launch_step(k_two<F>, sh.grid, sh.block, st, ps, pd, s.g, K);
 }
 
 cudaError_t launch_step_out_of_place(const Lattice& src, const Lattice& dst, double omega, cudaStream_t st) {
@@ -1630,13 +1670,11 @@ cudaError_t launch_step_out_of_place(const Lattice& src, const Lattice& dst, dou
   const Shape sh = cell_shape(src.g);
   switch (src.form) {
     case FORM_F64:
-      k_two<F64><<<sh.grid, sh.block, 0, st>>>(pops_of<const double>(src), pops_of<double>(dst), src.g, K);
-      return cudaGetLastError();
+      return launch_step(k_two<F64>, sh.grid, sh.block, st, pops_of<const double>(src), pops_of<double>(dst), src.g, K);
     case FORM_F32: {
       const VecRows r(src.g, 2, true);
-      launch_vec(k_two_f32v<false, false>, k_two_f32v<false, true>, src.g, r, src.g.nz, st, pops_of<const float>(src),
+      return launch_vec(k_two_f32v<false, false>, k_two_f32v<false, true>, src.g, r, src.g.nz, st, pops_of<const float>(src),
                  pops_of<float>(dst), src.g, K, r.arg, 0);
-      return cudaGetLastError();
     }
   }
   return cudaErrorInvalidValue;
@@ -1668,16 +1706,15 @@ static cudaError_t aa_impl(const Lattice& a, int odd, const StepK& K, int varian
     const Pops<float> pf = pops_of<float>(a);
     const VecRows r4(a.g, 4, false, true), r(a.g, 2, false);
     if (odd && variant == 0 && r4.arg >= 0) {
-      if (K.les) launch_vec(k_aa_f32w<true, false>, k_aa_f32w<true, true>, a.g, r4, a.g.nz, st, pf, a.g, K, r4.arg);
-      else launch_vec(k_aa_f32w<false, false>, k_aa_f32w<false, true>, a.g, r4, a.g.nz, st, pf, a.g, K, r4.arg);
+      if (K.les) return launch_vec(k_aa_f32w<true, false>, k_aa_f32w<true, true>, a.g, r4, a.g.nz, st, pf, a.g, K, r4.arg);
+      else return launch_vec(k_aa_f32w<false, false>, k_aa_f32w<false, true>, a.g, r4, a.g.nz, st, pf, a.g, K, r4.arg);
     } else if (K.les) {
-      if (odd) launch_vec(k_aa_f32v<true, true, false>, k_aa_f32v<true, true, true>, a.g, r, a.g.nz, st, pf, a.g, K, r.arg);
-      else launch_vec(k_aa_f32v<false, true, false>, k_aa_f32v<false, true, true>, a.g, r, a.g.nz, st, pf, a.g, K, r.arg);
+      if (odd) return launch_vec(k_aa_f32v<true, true, false>, k_aa_f32v<true, true, true>, a.g, r, a.g.nz, st, pf, a.g, K, r.arg);
+      else return launch_vec(k_aa_f32v<false, true, false>, k_aa_f32v<false, true, true>, a.g, r, a.g.nz, st, pf, a.g, K, r.arg);
     } else {
-      if (odd) launch_vec(k_aa_f32v<true, false, false>, k_aa_f32v<true, false, true>, a.g, r, a.g.nz, st, pf, a.g, K, r.arg);
-      else launch_vec(k_aa_f32v<false, false, false>, k_aa_f32v<false, false, true>, a.g, r, a.g.nz, st, pf, a.g, K, r.arg);
+      if (odd) return launch_vec(k_aa_f32v<true, false, false>, k_aa_f32v<true, false, true>, a.g, r, a.g.nz, st, pf, a.g, K, r.arg);
+      else return launch_vec(k_aa_f32v<false, false, false>, k_aa_f32v<false, false, true>, a.g, r, a.g.nz, st, pf, a.g, K, r.arg);
     }
-    return cudaGetLastError();
   }
   // FP16 (automatic or 4): four cells per thread. The automatic BGK odd step has
   // eight where rows are whole chunks: on B200 the pair of AA steps measured
@@ -1690,20 +1727,18 @@ static cudaError_t aa_impl(const Lattice& a, int odd, const StepK& K, int varian
     const Pops<__half> ph = pops_of<__half>(a);
     const VecRows r8(a.g, 8, false, true), r(a.g, 4, false);
     if (K.les) {
-      if (odd) launch_vec(k_aa_f16v<true, true, false>, k_aa_f16v<true, true, true>, a.g, r, a.g.nz, st, ph, a.g, K, r.arg);
-      else launch_vec(k_aa_f16v<false, true, false>, k_aa_f16v<false, true, true>, a.g, r, a.g.nz, st, ph, a.g, K, r.arg);
+      if (odd) return launch_vec(k_aa_f16v<true, true, false>, k_aa_f16v<true, true, true>, a.g, r, a.g.nz, st, ph, a.g, K, r.arg);
+      else return launch_vec(k_aa_f16v<false, true, false>, k_aa_f16v<false, true, true>, a.g, r, a.g.nz, st, ph, a.g, K, r.arg);
     } else if (odd && variant == 0 && r8.arg >= 0) {
-      launch_vec(k_aa_f16w<true, false>, k_aa_f16w<true, true>, a.g, r8, a.g.nz, st, ph, a.g, K, r8.arg);
+      return launch_vec(k_aa_f16w<true, false>, k_aa_f16w<true, true>, a.g, r8, a.g.nz, st, ph, a.g, K, r8.arg);
     } else {
-      if (odd) launch_vec(k_aa_f16v<true, false, false>, k_aa_f16v<true, false, true>, a.g, r, a.g.nz, st, ph, a.g, K, r.arg);
-      else launch_vec(k_aa_f16v<false, false, false>, k_aa_f16v<false, false, true>, a.g, r, a.g.nz, st, ph, a.g, K, r.arg);
+      if (odd) return launch_vec(k_aa_f16v<true, false, false>, k_aa_f16v<true, false, true>, a.g, r, a.g.nz, st, ph, a.g, K, r.arg);
+      else return launch_vec(k_aa_f16v<false, false, false>, k_aa_f16v<false, false, true>, a.g, r, a.g.nz, st, ph, a.g, K, r.arg);
     }
-    return cudaGetLastError();
   }
   if (K.les) {
-    if (odd) k_aa<F, true, true><<<sh.grid, sh.block, 0, st>>>(pops_of<S>(a), a.g, K);
-    else k_aa<F, false, true><<<sh.grid, sh.block, 0, st>>>(pops_of<S>(a), a.g, K);
-    return cudaGetLastError();
+    if (odd) return launch_step(k_aa<F, true, true>, sh.grid, sh.block, st, pops_of<S>(a), a.g, K);
+    else return launch_step(k_aa<F, false, true>, sh.grid, sh.block, st, pops_of<S>(a), a.g, K);
   }
   if (variant == 8) {
     bool launched = false;
@@ -1711,10 +1746,9 @@ static cudaError_t aa_impl(const Lattice& a, int odd, const StepK& K, int varian
     if (e != cudaSuccess || launched) return e;
   }
   if (odd && F::id == FORM_F16)
-    k_aa_f16_odd<<<sh.grid, sh.block, 0, st>>>(pops_of<__half>(a), a.g, K);
-  else if (odd) k_aa<F, true><<<sh.grid, sh.block, 0, st>>>(pops_of<S>(a), a.g, K);
-  else k_aa<F, false><<<sh.grid, sh.block, 0, st>>>(pops_of<S>(a), a.g, K);
-  return cudaGetLastError();
+    return launch_step(k_aa_f16_odd, sh.grid, sh.block, st, pops_of<__half>(a), a.g, K);
+  else if (odd) return launch_step(k_aa<F, true>, sh.grid, sh.block, st, pops_of<S>(a), a.g, K);
+  else return launch_step(k_aa<F, false>, sh.grid, sh.block, st, pops_of<S>(a), a.g, K);
 }
 
 cudaError_t launch_aa(const Lattice& a, int odd, double omega, double scale, double les_cs, int variant,
@@ -1918,14 +1952,14 @@ static cudaError_t slab_impl(const Lattice& s, const Lattice& d, const StepK& K,
       Pops<float> pf = pops_of<float>(d);
       pf.p[Q - 1] = (float*)s.p[Q - 1];
       const VecRows r(s.g, 2, true);
-      if (K.les) launch_vec(k_two_f32v<true, false>, k_two_f32v<true, true>, s.g, r, ni, st_in, pops_of<const float>(s), pf, s.g, K, r.arg, 1);
-      else launch_vec(k_two_f32v<false, false>, k_two_f32v<false, true>, s.g, r, ni, st_in, pops_of<const float>(s), pf, s.g, K, r.arg, 1);
+      if (K.les) launch_vec_plain(k_two_f32v<true, false>, k_two_f32v<true, true>, s.g, r, ni, st_in, pops_of<const float>(s), pf, s.g, K, r.arg, 1);
+      else launch_vec_plain(k_two_f32v<false, false>, k_two_f32v<false, true>, s.g, r, ni, st_in, pops_of<const float>(s), pf, s.g, K, r.arg, 1);
     } else if (F::id == FORM_F16) {
       Pops<__half> ph = pops_of<__half>(d);
       ph.p[Q - 1] = (__half*)s.p[Q - 1];
       const VecRows r(s.g, 4, true);
-      if (K.les) launch_vec(k_two_f16v<true, false>, k_two_f16v<true, true>, s.g, r, ni, st_in, pops_of<const __half>(s), ph, s.g, K, r.arg, 1);
-      else launch_vec(k_two_f16v<false, false>, k_two_f16v<false, true>, s.g, r, ni, st_in, pops_of<const __half>(s), ph, s.g, K, r.arg, 1);
+      if (K.les) launch_vec_plain(k_two_f16v<true, false>, k_two_f16v<true, true>, s.g, r, ni, st_in, pops_of<const __half>(s), ph, s.g, K, r.arg, 1);
+      else launch_vec_plain(k_two_f16v<false, false>, k_two_f16v<false, true>, s.g, r, ni, st_in, pops_of<const __half>(s), ph, s.g, K, r.arg, 1);
     } else {
       const dim3 gi(sh.grid.x, sh.grid.y, s.g.nz - 2);
       if (K.les) k_slab<F, true, false><<<gi, sh.block, 0, st_in>>>(ps, pd, s.g, K, h);
