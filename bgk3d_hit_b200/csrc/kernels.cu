@@ -1250,8 +1250,14 @@ __global__ void k_faith_snapshot(Pops<const S> a, Geo g, S* out) {
 enum { PULL_WRAP = 0, PULL_SLAB = 1, PULL_FAITH = 2 };
 constexpr int NDK = 9;  // quantities of k_diag
 
+// Blocks of k_diag: what the SMs hold at once (128 registers in FP64, 80 in the
+// others), so that no second wave runs half empty. 256^3, us, with 592 blocks and
+// so: FP64 727 / 659, FP32 644 / 510, FP16 602 / 513.
+__host__ __device__ constexpr int diag_blocks_per_sm(int form) { return form == FORM_F64 ? 2 : 3; }
+static int diag_blocks(int form) { return 148 * diag_blocks_per_sm(form); }
+
 template <class F, int LAY, int PULL>
-__global__ void __launch_bounds__(DIAG_THREADS, F::id == 0 ? 2 : 3)
+__global__ void __launch_bounds__(DIAG_THREADS, diag_blocks_per_sm(F::id))
     k_diag(Pops<const typename F::S> a, Geo g, double svisc, double omega, typename F::R inv, double* partials,
            typename F::R* vel, Halo<typename F::S> h, const typename F::S* __restrict__ faith, int faith_zero) {
   using R = typename F::R; using V = typename F::V; using N = Num<V>;
@@ -1316,9 +1322,10 @@ __global__ void __launch_bounds__(DIAG_THREADS, F::id == 0 ? 2 : 3)
   }
   acc[8].s = (double)bad;
   const KS r = block_reduce_n<NDK, DIAG_THREADS>(acc, sh);
-  if (threadIdx.x < NDK) {
-    partials[(blockIdx.x * ND + threadIdx.x) * 2 + 0] = r.s;
-    partials[(blockIdx.x * ND + threadIdx.x) * 2 + 1] = r.c;
+  constexpr int W = DIAG_THREADS / 32;
+  if (threadIdx.x % W == 0 && threadIdx.x / W < NDK) {
+    partials[(blockIdx.x * ND + threadIdx.x / W) * 2 + 0] = r.s;
+    partials[(blockIdx.x * ND + threadIdx.x / W) * 2 + 1] = r.c;
   }
 }
 
@@ -1351,7 +1358,7 @@ __global__ void __launch_bounds__(256) k_velocity(Pops<const typename F::S> a, G
 
 template <class R>
 __global__ void __launch_bounds__(DIAG_THREADS) k_enstrophy(const R* __restrict__ vel, int nx, int ny, int nz,
-                                                            double* partials) {
+                                                           double* partials) {
   __shared__ KS sh[DIAG_THREADS / 32][1];
   KS acc[1] = {{0.0, 0.0}};
   const long long n = (long long)nx * ny * nz;
@@ -1388,12 +1395,13 @@ __global__ void __launch_bounds__(DIAG_THREADS) k_enstrophy(const R* __restrict_
 // One block per quantity (one block for all ten took 16 us). totals may be
 // pinned host memory; err (optional): the device's error flag, copied behind
 // the ND + 1 totals so that the host reads one place.
-__global__ void __launch_bounds__(DIAG_THREADS) k_finalize(const double* __restrict__ partials, double* totals,
-                                                           const int* err) {
+__global__ void __launch_bounds__(DIAG_THREADS) k_finalize(const double* __restrict__ partials, int blocks,
+                                                           double* totals, const int* err) {
   __shared__ KS sh[DIAG_THREADS / 32][1];
   const int d = blockIdx.x;
   KS acc[1] = {{0.0, 0.0}};
-  for (int b = threadIdx.x; b < DIAG_BLOCKS; b += blockDim.x) {
+  const int nb = d < NDK ? blocks : DIAG_BLOCKS;  // k_diag's, k_enstrophy's
+  for (int b = threadIdx.x; b < nb; b += blockDim.x) {
     const double2 p = __ldg(reinterpret_cast<const double2*>(partials) + b * ND + d);
     kcomb(acc[0], KS{p.x, p.y});
   }
@@ -1862,7 +1870,7 @@ template <class F, int LAY, int PULL>
 static void diag_pull(const Lattice& a, double svisc, double omega, double scale, double* partials, void* vel,
                       const SlabLinks* halo, const void* faith, bool fzero, cudaStream_t st) {
   using S = typename F::S; using R = typename F::R;
-  k_diag<F, LAY, PULL><<<DIAG_BLOCKS, DIAG_THREADS, 0, st>>>(pops_of<const S>(a), a.g, svisc, omega, (R)(1.0 / scale),
+  k_diag<F, LAY, PULL><<<diag_blocks(F::id), DIAG_THREADS, 0, st>>>(pops_of<const S>(a), a.g, svisc, omega, (R)(1.0 / scale),
                                                             partials, (R*)vel, halo_of<S>(halo), (const S*)faith,
                                                             fzero ? 1 : 0);
 }
@@ -2004,8 +2012,9 @@ cudaError_t launch_enstrophy(const Lattice& a, const void* vel, double* partials
   return cudaGetLastError();
 }
 
-cudaError_t launch_finalize(const double* partials, double* totals, cudaStream_t st, const int* err) {
-  k_finalize<<<ND, DIAG_THREADS, 0, st>>>(partials, totals, err);
+cudaError_t launch_finalize(const double* partials, int form, bool enstrophy, double* totals, cudaStream_t st,
+                            const int* err) {
+  k_finalize<<<enstrophy ? ND : NDK, DIAG_THREADS, 0, st>>>(partials, diag_blocks(form), totals, err);
   return cudaGetLastError();
 }
 

@@ -140,9 +140,12 @@ cudaError_t launch_enstrophy(const Lattice& a, const void* vel, double* partials
 // as double or in the form's arithmetic type), nothing else.
 cudaError_t launch_velocity(const Lattice& a, int lay, double scale, void* vel, bool as_double, int k0, int nk,
                             cudaStream_t st);
-// Sums DIAG_BLOCKS partials into ND totals (fixed order, compensated); with
-// err, also the error flag as totals[ND + 1]. totals: device or pinned host.
-cudaError_t launch_finalize(const double* partials, double* totals, cudaStream_t st, const int* err = nullptr);
+// Sums the partials of a form's launch_diag (and, with enstrophy, of
+// launch_enstrophy) into the totals of the ND quantities (fixed order,
+// compensated); with err, also the error flag as totals[ND + 1]. totals: device or
+// pinned host.
+cudaError_t launch_finalize(const double* partials, int form, bool enstrophy, double* totals, cudaStream_t st,
+                            const int* err = nullptr);
 // Faithful-mode helper: zj of the last cell (i=l, j=m, k=n) into *out.
 cudaError_t launch_last_zj(const Lattice& a, int lay, double scale, double* out, cudaStream_t st);
 

@@ -101,7 +101,7 @@ extern "C" int bgk_diagnostics_noalloc(const void* const* pops19, int lx, int ly
   // Every partial slot and every total is written by these kernels before it
   // is read, so nothing left from an earlier call has to be cleared.
   cudaError_t e = launch_diag(lat, LAY_TWO, svisc, omega, scale, partials, nullptr, st);
-  if (e == cudaSuccess) e = launch_finalize(partials, totals, st);
+  if (e == cudaSuccess) e = launch_finalize(partials, precision, false, totals, st);
   if (e == cudaSuccess && faithful) e = launch_last_zj(lat, LAY_TWO, scale, totals + ND, st);
   double t[ND + 1] = {0};
   if (e == cudaSuccess) e = cudaMemcpyAsync(t, totals, sizeof(t), cudaMemcpyDeviceToHost, st);

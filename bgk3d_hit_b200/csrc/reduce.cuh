@@ -35,13 +35,13 @@ __device__ __forceinline__ KS block_reduce(KS v, KS* sh) {
   return r;
 }
 
-// The same for N quantities at once: shuffles inside the warps, then one thread
-// per quantity over the warps' pairs, so a block pays two barriers instead of
+// The same for N quantities at once: shuffles inside the warps, then shuffles over
+// the warps' pairs, so a block pays two barriers instead of
 // a shared-memory tree per quantity (nine of them were 9 us of the 22 us that
-// the diagnostics of a 32^3 box took). Thread d < N returns quantity d.
+// the diagnostics of a 32^3 box took). Thread d * THREADS / 32 returns quantity d.
 template <int N, int THREADS>
 __device__ __forceinline__ KS block_reduce_n(KS (&v)[N], KS (&sh)[THREADS / 32][N]) {
-  static_assert(THREADS % 32 == 0 && N <= THREADS, "whole warps");
+  static_assert(THREADS % 32 == 0 && N * (THREADS / 32) <= THREADS && 32 % (THREADS / 32) == 0, "whole warps");
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll
   for (int d = 0; d < N; ++d) {
@@ -53,10 +53,16 @@ __device__ __forceinline__ KS block_reduce_n(KS (&v)[N], KS (&sh)[THREADS / 32][
     if (lane == 0) sh[w][d] = v[d];
   }
   __syncthreads();
+  // W threads per quantity and a tree again: thread d * W returns quantity d
+  constexpr int W = THREADS / 32;
   KS r = {0.0, 0.0};
-  if (threadIdx.x < N) {
-    r = sh[0][threadIdx.x];
-    for (int m = 1; m < THREADS / 32; ++m) kcomb(r, sh[m][threadIdx.x]);
+  if (threadIdx.x < (N * W + 31) / 32 * 32) {
+    if (threadIdx.x < N * W) r = sh[threadIdx.x % W][threadIdx.x / W];
+#pragma unroll
+    for (int s = W / 2; s > 0; s >>= 1) {
+      const KS o = {__shfl_down_sync(0xffffffffu, r.s, s, W), __shfl_down_sync(0xffffffffu, r.c, s, W)};
+      kcomb(r, o);
+    }
   }
   return r;
 }
