@@ -1352,6 +1352,7 @@ struct AdjBufs {
     void* m = c->lat_pool[next++];
     L->form = c->form;
     L->g = c->g;
+    L->err = c->d_err;
     for (int q = 0; q < Q; ++q) L->p[q] = (char*)m + (size_t)q * c->g.qs * c->es;
     return BGK_OK;
   }
@@ -1484,22 +1485,31 @@ int bgk_adjoint(bgk_ctx* c, const double* u0, const double* v0, const double* w0
   CK(launch_init_velocity(ck[0], LAY_TWO, du0, du0 + n, du0 + 2 * n, 1.0, 0, c->g.nz, 1.0, nullptr, c->st));
   const Lattice* cur = &ck[0];
   int wi = 0;
-  for (int t = 0; t < T; ++t) {
-    const Lattice* next;
-    const int s = t / K, m = t + 1 - s * K;  // f^{t+1} is state m of segment s
-    if (want_grad && t + 1 < T && (t + 1) % K == 0) next = &ck[(t + 1) / K];
-    else if (want_grad && s >= s_cache && t + 1 < T) next = &cache[s][m - 1];
-    else {
+  // where f^t is kept for the backward pass, or null
+  auto kept = [&](int t) -> const Lattice* {
+    if (!want_grad || t >= T) return nullptr;
+    if (t % K == 0) return &ck[t / K];
+    return t / K >= s_cache ? &cache[t / K][t % K - 1] : nullptr;
+  };
+  // a state that nobody keeps is passed over where two steps per launch pay
+  const bool pairs = two_steps_pay(c->g, c->form, false);
+  for (int t = 0; t < T;) {
+    const int n = pairs && t + 2 <= T && !kept(t + 1) ? 2 : 1;
+    const Lattice* next = kept(t + n);
+    if (!next) {
       if (cur == &work[wi]) wi ^= 1;
       next = &work[wi];
     }
-    CK(launch_step_out_of_place(*cur, *next, c->omega, c->st));
+    if (n == 2) CK(launch_two_steps(*cur, *next, c->omega, 1.0, 0.0, c->st));
+    else CK(launch_step_out_of_place(*cur, *next, c->omega, c->st));
+    c->launches++;
     cur = next;
+    t += n;
   }
   CK(cudaMemsetAsync(acc, 0, 2 * DIAG_BLOCKS * sizeof(double), c->st));
   CK(launch_adj_terminal(*cur, dut, lam[0], acc, c->st));
   CK(launch_acc_total(acc, tot, c->st));
-  c->launches += T + 3;
+  c->launches += 3;
   if (want_grad) {
     // backward over the segments, recomputing each from its checkpoint
     CK(cudaMemsetAsync(acc, 0, 2 * nacc * sizeof(double), c->st));
@@ -1549,7 +1559,7 @@ int bgk_adjoint(bgk_ctx* c, const double* u0, const double* v0, const double* w0
   }
   double h[2] = {0.0, 0.0};
   CK(cudaMemcpyAsync(h, tot, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->st));
-  CK(cudaStreamSynchronize(c->st));
+  if ((rc = sync_and_check(c))) return rc;
   *loss = h[0] / (double)n;
   if (grad_tau) *grad_tau = -c->omega * c->omega * h[1];  // tau = 1/omega
   return BGK_OK;

@@ -76,3 +76,27 @@ def test_fused_and_single_steps_mixed(bgk):
     assert _same(ref, box)
     ref.close()
     box.close()
+
+
+@pytest.mark.parametrize("steps", [4, 7])
+def test_adjoint_forward_in_pairs(bgk, steps):
+    """States that no checkpoint keeps are passed over two steps at a time; with a
+    checkpoint at every step none are. The results are the same bits."""
+    import ctypes as C
+
+    nx, ny, nz = shape = (128, 128, 128)
+    rng = np.random.default_rng(2)
+    u = [np.ascontiguousarray(0.03 * rng.standard_normal((nz, ny, nx))) for _ in range(6)]
+    dp = C.POINTER(C.c_double)
+    box = bgk.BGK3D(*shape, svisc=0.03)
+    got = []
+    for every in (1, 3, 7):
+        loss, gtau, grad = C.c_double(), C.c_double(), np.zeros((3, nz, ny, nx))
+        rc = box._lib.bgk_adjoint(box._h, *(a.ctypes.data_as(dp) for a in u), steps, every, C.byref(loss),
+                                  grad.ctypes.data_as(dp), C.byref(gtau))
+        assert rc == 0
+        got.append((loss.value, gtau.value, grad))
+    for loss, gtau, grad in got[1:]:
+        assert loss == got[0][0] and gtau == got[0][1]
+        assert np.array_equal(grad, got[0][2])
+    box.close()
