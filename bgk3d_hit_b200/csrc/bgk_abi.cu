@@ -404,7 +404,7 @@ int compute_diag(bgk_ctx* c, int itime, bgk_diag* out, int want_extras) {
     faith = faith_buf(c, c->step);
   }
   CK(launch_diag(c->A, c->lay, c->p.svisc, c->omega, c->scale, c->partials, extras ? c->vel : nullptr, c->st,
-                 c->slab ? &hl : nullptr, faith, faith_zero));
+                 c->slab ? &hl : nullptr, faith, faith_zero, !c->slab));
   c->launches++;
   if (extras) {
     CK(launch_enstrophy(c->A, c->vel, c->partials, c->st));
@@ -412,7 +412,7 @@ int compute_diag(bgk_ctx* c, int itime, bgk_diag* out, int want_extras) {
   }
   // the totals and the error flag go straight to pinned host memory: no copies
   // behind the kernels (two of them were a tenth of a 32^3 box's diagnostics)
-  CK(launch_finalize(c->partials, c->form, extras, c->h_tot, c->st, c->d_err));
+  CK(launch_finalize(c->partials, c->form, extras, c->h_tot, c->st, c->d_err, true));
   c->launches++;
   const bool faithful = c->p.mode == BGK_FAITHFUL;
   if (faithful) {

@@ -73,10 +73,12 @@ static Shape cell_shape(const Geo& g) {
   return s;
 }
 
-// Launches a step kernel so that it may be scheduled beside the end of the kernel
-// before it in the stream (see step_begin).
+// Launches a kernel that starts with step_begin; overlap: so that it may be scheduled
+// beside the end of the kernel before it in the stream. Only on a context's own
+// stream, where that kernel is one of these or an ordinary one: step_begin waits
+// for the kernel before, and through its own for those before that.
 template <class... P, class... A>
-static cudaError_t launch_step(void (*kern)(P...), dim3 grid, dim3 block, cudaStream_t st, A... args) {
+static cudaError_t launch_after(bool overlap, void (*kern)(P...), dim3 grid, dim3 block, cudaStream_t st, A... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -85,8 +87,12 @@ static cudaError_t launch_step(void (*kern)(P...), dim3 grid, dim3 block, cudaSt
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = overlap ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
+template <class... P, class... A>
+static cudaError_t launch_step(void (*kern)(P...), dim3 grid, dim3 block, cudaStream_t st, A... args) {
+  return launch_after(true, kern, grid, block, st, args...);
 }
 
 static int grid_1d(long long n, int threads, int cap) {
@@ -1260,6 +1266,7 @@ template <class F, int LAY, int PULL>
 __global__ void __launch_bounds__(DIAG_THREADS, diag_blocks_per_sm(F::id))
     k_diag(Pops<const typename F::S> a, Geo g, double svisc, double omega, typename F::R inv, double* partials,
            typename F::R* vel, Halo<typename F::S> h, const typename F::S* __restrict__ faith, int faith_zero) {
+  step_begin();
   using R = typename F::R; using V = typename F::V; using N = Num<V>;
   __shared__ KS sh[DIAG_THREADS / 32][NDK];
   KS acc[NDK];
@@ -1359,6 +1366,7 @@ __global__ void __launch_bounds__(256) k_velocity(Pops<const typename F::S> a, G
 template <class R>
 __global__ void __launch_bounds__(DIAG_THREADS) k_enstrophy(const R* __restrict__ vel, int nx, int ny, int nz,
                                                            double* partials) {
+  step_begin();
   __shared__ KS sh[DIAG_THREADS / 32][1];
   KS acc[1] = {{0.0, 0.0}};
   const long long n = (long long)nx * ny * nz;
@@ -1397,6 +1405,7 @@ __global__ void __launch_bounds__(DIAG_THREADS) k_enstrophy(const R* __restrict_
 // the ND + 1 totals so that the host reads one place.
 __global__ void __launch_bounds__(DIAG_THREADS) k_finalize(const double* __restrict__ partials, int blocks,
                                                            double* totals, const int* err) {
+  step_begin();
   __shared__ KS sh[DIAG_THREADS / 32][1];
   const int d = blockIdx.x;
   KS acc[1] = {{0.0, 0.0}};
@@ -1867,22 +1876,21 @@ template <class S> static Halo<S> halo_of(const SlabLinks* l) {
 }
 
 template <class F, int LAY, int PULL>
-static void diag_pull(const Lattice& a, double svisc, double omega, double scale, double* partials, void* vel,
+static cudaError_t diag_pull(bool overlap, const Lattice& a, double svisc, double omega, double scale, double* partials, void* vel,
                       const SlabLinks* halo, const void* faith, bool fzero, cudaStream_t st) {
   using S = typename F::S; using R = typename F::R;
-  k_diag<F, LAY, PULL><<<diag_blocks(F::id), DIAG_THREADS, 0, st>>>(pops_of<const S>(a), a.g, svisc, omega, (R)(1.0 / scale),
-                                                            partials, (R*)vel, halo_of<S>(halo), (const S*)faith,
-                                                            fzero ? 1 : 0);
+  return launch_after(overlap, k_diag<F, LAY, PULL>, diag_blocks(F::id), DIAG_THREADS, st, pops_of<const S>(a), a.g,
+                      svisc, omega, (R)(1.0 / scale), partials, (R*)vel, halo_of<S>(halo), (const S*)faith,
+                      fzero ? 1 : 0);
 }
 template <class F>
-static cudaError_t diag_impl(const Lattice& a, int lay, double svisc, double omega, double scale, double* partials,
+static cudaError_t diag_impl(bool overlap, const Lattice& a, int lay, double svisc, double omega, double scale, double* partials,
                              void* vel, const SlabLinks* halo, const void* faith, bool fzero, cudaStream_t st) {
-  if (lay == LAY_AAE) diag_pull<F, LAY_AAE, PULL_WRAP>(a, svisc, omega, scale, partials, vel, nullptr, nullptr, false, st);
-  else if (lay == LAY_AAN) diag_pull<F, LAY_AAN, PULL_WRAP>(a, svisc, omega, scale, partials, vel, nullptr, nullptr, false, st);
-  else if (halo) diag_pull<F, LAY_TWO, PULL_SLAB>(a, svisc, omega, scale, partials, vel, halo, nullptr, false, st);
-  else if (faith || fzero) diag_pull<F, LAY_TWO, PULL_FAITH>(a, svisc, omega, scale, partials, vel, nullptr, faith, fzero, st);
-  else diag_pull<F, LAY_TWO, PULL_WRAP>(a, svisc, omega, scale, partials, vel, nullptr, nullptr, false, st);
-  return cudaGetLastError();
+  if (lay == LAY_AAE) return diag_pull<F, LAY_AAE, PULL_WRAP>(overlap, a, svisc, omega, scale, partials, vel, nullptr, nullptr, false, st);
+  if (lay == LAY_AAN) return diag_pull<F, LAY_AAN, PULL_WRAP>(overlap, a, svisc, omega, scale, partials, vel, nullptr, nullptr, false, st);
+  if (halo) return diag_pull<F, LAY_TWO, PULL_SLAB>(overlap, a, svisc, omega, scale, partials, vel, halo, nullptr, false, st);
+  if (faith || fzero) return diag_pull<F, LAY_TWO, PULL_FAITH>(overlap, a, svisc, omega, scale, partials, vel, nullptr, faith, fzero, st);
+  return diag_pull<F, LAY_TWO, PULL_WRAP>(overlap, a, svisc, omega, scale, partials, vel, nullptr, nullptr, false, st);
 }
 
 template <class F, class OUT>
@@ -1927,11 +1935,12 @@ cudaError_t launch_faith_snapshot(const Lattice& a, void* out, cudaStream_t st) 
   return cudaGetLastError();
 }
 cudaError_t launch_diag(const Lattice& a, int lay, double svisc, double omega, double scale, double* partials,
-                        void* vel, cudaStream_t st, const SlabLinks* halo, const void* faith, bool faith_zero) {
+                        void* vel, cudaStream_t st, const SlabLinks* halo, const void* faith, bool faith_zero,
+                        bool overlap) {
   switch (a.form) {
-    case FORM_F64: return diag_impl<F64>(a, lay, svisc, omega, scale, partials, vel, halo, faith, faith_zero, st);
-    case FORM_F32: return diag_impl<F32>(a, lay, svisc, omega, scale, partials, vel, halo, faith, faith_zero, st);
-    case FORM_F16: return diag_impl<F16>(a, lay, svisc, omega, scale, partials, vel, halo, faith, faith_zero, st);
+    case FORM_F64: return diag_impl<F64>(overlap, a, lay, svisc, omega, scale, partials, vel, halo, faith, faith_zero, st);
+    case FORM_F32: return diag_impl<F32>(overlap, a, lay, svisc, omega, scale, partials, vel, halo, faith, faith_zero, st);
+    case FORM_F16: return diag_impl<F16>(overlap, a, lay, svisc, omega, scale, partials, vel, halo, faith, faith_zero, st);
   }
   return cudaErrorInvalidValue;
 }
@@ -2006,16 +2015,13 @@ cudaError_t launch_halo_prime(const Lattice& a, const SlabLinks& links, cudaStre
 
 cudaError_t launch_enstrophy(const Lattice& a, const void* vel, double* partials, cudaStream_t st) {
   if (a.form == FORM_F64)
-    k_enstrophy<double><<<DIAG_BLOCKS, DIAG_THREADS, 0, st>>>((const double*)vel, a.g.nx, a.g.ny, a.g.nz, partials);
-  else
-    k_enstrophy<float><<<DIAG_BLOCKS, DIAG_THREADS, 0, st>>>((const float*)vel, a.g.nx, a.g.ny, a.g.nz, partials);
-  return cudaGetLastError();
+    return launch_step(k_enstrophy<double>, DIAG_BLOCKS, DIAG_THREADS, st, (const double*)vel, a.g.nx, a.g.ny, a.g.nz, partials);
+  return launch_step(k_enstrophy<float>, DIAG_BLOCKS, DIAG_THREADS, st, (const float*)vel, a.g.nx, a.g.ny, a.g.nz, partials);
 }
 
 cudaError_t launch_finalize(const double* partials, int form, bool enstrophy, double* totals, cudaStream_t st,
-                            const int* err) {
-  k_finalize<<<enstrophy ? ND : NDK, DIAG_THREADS, 0, st>>>(partials, diag_blocks(form), totals, err);
-  return cudaGetLastError();
+                            const int* err, bool overlap) {
+  return launch_after(overlap, k_finalize, enstrophy ? ND : NDK, DIAG_THREADS, st, partials, diag_blocks(form), totals, err);
 }
 
 template <class F>

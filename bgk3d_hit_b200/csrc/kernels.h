@@ -117,7 +117,8 @@ cudaError_t launch_import(const Lattice& a, int lay, int q0, int nq, const void*
 long long faith_planes_elems(const Geo& g);
 cudaError_t launch_faith_snapshot(const Lattice& a, void* out, cudaStream_t st);
 
-// Diagnostics: per-block partial sums (Neumaier pairs) of ND quantities.
+// Diagnostics (overlap: launched beside the end of the kernel before, on a
+// context's own stream): per-block partial sums (Neumaier pairs) of ND quantities.
 // vel (optional, 3*N values of the arithmetic type) receives the local velocity.
 // halo: the ghost planes of a z-slab (in_lo / in_hi), nullptr for a whole box.
 // faith (two-lattice only): pulls that leave the box read the periodic image
@@ -125,7 +126,7 @@ cudaError_t launch_faith_snapshot(const Lattice& a, void* out, cudaStream_t st);
 // faith_zero they read a zero deviation (ghosts never written).
 cudaError_t launch_diag(const Lattice& a, int lay, double svisc, double omega, double scale, double* partials,
                         void* vel, cudaStream_t st, const SlabLinks* halo = nullptr, const void* faith = nullptr,
-                        bool faith_zero = false);
+                        bool faith_zero = false, bool overlap = false);
 
 // z-slab two-lattice step (src -> dst, pop 19 in place) reading the ghost
 // planes links.in_* and storing the outgoing boundary populations into
@@ -145,7 +146,7 @@ cudaError_t launch_velocity(const Lattice& a, int lay, double scale, void* vel, 
 // compensated); with err, also the error flag as totals[ND + 1]. totals: device or
 // pinned host.
 cudaError_t launch_finalize(const double* partials, int form, bool enstrophy, double* totals, cudaStream_t st,
-                            const int* err = nullptr);
+                            const int* err = nullptr, bool overlap = false);
 // Faithful-mode helper: zj of the last cell (i=l, j=m, k=n) into *out.
 cudaError_t launch_last_zj(const Lattice& a, int lay, double scale, double* out, cudaStream_t st);
 
