@@ -45,8 +45,8 @@ constexpr int MAX_POLLS = 1 << 20;
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 // Bounded: false when the copies did not land.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-  for (int n = 0; n < MAX_POLLS; ++n) {
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int polls) {
+  for (int n = 0; n < polls; ++n) {
     uint32_t done;
     asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n}\n"
                  : "=r"(done)
@@ -214,8 +214,8 @@ __global__ void __launch_bounds__(Two2<typename F::S, TY>::THREADS, 1)
     bool dead = false;
     for (int k = 0; k < np; ++k) {
       S* const raw = &sm.raw[k & 1][0][0];
-      if (!dead && !mbar_wait(smem_u32(&sm.bar[k & 1]), (k >> 1) & 1)) {
-        dead = true;  // reported; the remaining waits are skipped
+      if (!mbar_wait(smem_u32(&sm.bar[k & 1]), (k >> 1) & 1, dead ? 1 << 10 : MAX_POLLS)) {
+        dead = true;  // reported; the remaining waits are short
         *err = 1;
       }
       if (yedge) {

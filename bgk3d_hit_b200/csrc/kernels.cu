@@ -484,7 +484,10 @@ __global__ void __launch_bounds__(128, 5) k_aa_f16v(Pops<__half> a, Geo g, StepK
     __syncthreads();
     if (!valid) return;
   }
-  int js = j, ks = k;  // store rows: recomputed after the collision (BGK odd step)
+  const auto as = at.again(g, rows);
+  const XLanes xs = FLAT ? XLanes(as, threadIdx.x & 31) : xl;
+  const EdgeWarps es = FLAT ? EdgeWarps(as) : ew;
+  int js = FLAT ? as.j : j, ks = k;  // store rows: recomputed after the collision (BGK odd step)
   if (ODD) asm volatile("" : "+r"(js), "+r"(ks));
   const int jms = js == 0 ? g.ny - 1 : js - 1, jps = js == g.ny - 1 ? 0 : js + 1;
   const int kms = ks == 0 ? g.nz - 1 : ks - 1, kps = ks == g.nz - 1 ? 0 : ks + 1;
@@ -498,9 +501,9 @@ __global__ void __launch_bounds__(128, 5) k_aa_f16v(Pops<__half> a, Geo g, StepK
     if (!ODD) {
       *reinterpret_cast<uint2*>(a.p[oppq(q)] + row(0, 0) + i0) = Y[q];
     } else {
-      const unsigned fp = cxq(q) > 0 && xl.edge_prev && ew.prev_in ? xs_last[ew.wprev][q] : 0u;
-      const unsigned fn = cxq(q) < 0 && xl.edge_next && ew.next_in ? xs_first[ew.wnext][q - 9] : 0u;
-      shift_out(Y[q], cxq(q), a.p[q] + row_out(cyq(q), czq(q)), at, xl, ew, fp, fn);
+      const unsigned fp = cxq(q) > 0 && xs.edge_prev && es.prev_in ? xs_last[es.wprev][q] : 0u;
+      const unsigned fn = cxq(q) < 0 && xs.edge_next && es.next_in ? xs_first[es.wnext][q - 9] : 0u;
+      shift_out(Y[q], cxq(q), a.p[q] + row_out(cyq(q), czq(q)), as, xs, es, fp, fn);
     }
   }
 }
@@ -639,7 +642,10 @@ __global__ void __launch_bounds__(128, 4) k_aa_f16w(Pops<__half> a, Geo g, StepK
     __syncthreads();
     if (!valid) return;
   }
-  int js = j, ks = k;
+  const auto as = at.again(g, rows);
+  const XLanes xs = FLAT ? XLanes(as, threadIdx.x & 31) : xl;
+  const EdgeWarps es = FLAT ? EdgeWarps(as) : ew;
+  int js = FLAT ? as.j : j, ks = k;
   if (ODD) asm volatile("" : "+r"(js), "+r"(ks));
   const int jms = js == 0 ? g.ny - 1 : js - 1, jps = js == g.ny - 1 ? 0 : js + 1;
   const int kms = ks == 0 ? g.nz - 1 : ks - 1, kps = ks == g.nz - 1 ? 0 : ks + 1;
@@ -653,9 +659,9 @@ __global__ void __launch_bounds__(128, 4) k_aa_f16w(Pops<__half> a, Geo g, StepK
     if (!ODD) {
       *reinterpret_cast<uint4*>(a.p[oppq(q)] + row(0, 0) + i0) = Y[q];
     } else {
-      const unsigned fp = cxq(q) > 0 && xl.edge_prev && ew.prev_in ? xs_last[ew.wprev][q] : 0u;
-      const unsigned fn = cxq(q) < 0 && xl.edge_next && ew.next_in ? xs_first[ew.wnext][q - 9] : 0u;
-      shift_out8(Y[q], cxq(q), a.p[q] + row_out(cyq(q), czq(q)), at, xl, ew, fp, fn);
+      const unsigned fp = cxq(q) > 0 && xs.edge_prev && es.prev_in ? xs_last[es.wprev][q] : 0u;
+      const unsigned fn = cxq(q) < 0 && xs.edge_next && es.next_in ? xs_first[es.wnext][q - 9] : 0u;
+      shift_out8(Y[q], cxq(q), a.p[q] + row_out(cyq(q), czq(q)), as, xs, es, fp, fn);
     }
   }
 }
@@ -1739,7 +1745,7 @@ static cudaError_t aa_impl(const Lattice& a, int odd, const StepK& K, int varian
   // per thread on both steps; eight cells on the even step as well measured the
   // same (84.1, 86.1), so the even step stays on k_aa_f16v, and eight cells gave
   // the Smagorinsky odd step nothing (76.0 against 76.2, issue-bound). Rows of no
-  // power of two: 384 x 256 x 256 79.8 against 56.4 on one cell per thread
+  // power of two: 384 x 256 x 256 85.1 against 56.4 on one cell per thread
   if (F::id == FORM_F16 && (variant == 4 || (variant == 0 && big))) {
     const Pops<__half> ph = pops_of<__half>(a);
     const VecRows r8(a.g, 8, false, true), r(a.g, 4, false);

@@ -66,8 +66,16 @@ template <int V, bool FLAT> struct VecPlace {
   int cells;               // cells of the row's last chunk
   bool valid;              // false: past the plane's last thread; j is clamped
   bool end;                // the row's last chunk with cells, or behind it
-  __device__ VecPlace(const Geo& g, int arg) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  __device__ VecPlace(const Geo& g, int arg) : VecPlace(g, arg, blockIdx.x * blockDim.x + threadIdx.x) {}
+  // The same once more, so that nothing of it stays in registers in between (flat
+  // rows: the aligned ones' decode is cheap to keep).
+  __device__ VecPlace again(const Geo& g, int arg) const {
+    if (!FLAT) return *this;
+    int t = blockIdx.x * blockDim.x + threadIdx.x;
+    asm volatile("" : "+r"(t));
+    return VecPlace(g, arg, t);
+  }
+  __device__ VecPlace(const Geo& g, int arg, int t) {
     if (FLAT) {
       tpr = arg;
       j = (int)((unsigned)t / (unsigned)tpr);
