@@ -21,7 +21,8 @@ CSRC = os.path.join(HERE, "csrc")
 INCLUDE = os.path.join(ROOT, "include")
 OUT = os.path.join(HERE, "libbgk3d.so")
 SOURCES = ["kernels.cu", "fused.cu", "rows.cu", "adjoint.cu", "bgk_abi.cu", "noalloc.cu"]
-HEADERS = ["lattice.cuh", "kernels.h", "reduce.cuh", "vec.cuh"]
+HEADERS = ["lattice.cuh", "kernels.h", "reduce.cuh", "vec.cuh",
+           "launch.cuh"]
 ARCH = "-gencode=arch=compute_100a,code=sm_100a"
 
 

@@ -26,6 +26,7 @@
 // cells, and accumulate their sums into one compensated pair per block, so
 // repeated runs give identical bits.
 #include "kernels.h"
+#include "launch.cuh"
 #include "reduce.cuh"
 
 namespace bgk {
@@ -109,6 +110,7 @@ template <class F>
 __global__ void __launch_bounds__(128, 4) k_adj_step(Pops<const typename F::S> ft, Pops<const typename F::S> lin,
                                                      Pops<typename F::S> lout, Geo g, typename F::R omega,
                                                      double* acc) {
+  step_begin();
   using S = typename F::S; using R = typename F::R;
   using D = R;  // arithmetic of the moment sums: the form's (double for FP64, float for FP32)
   __shared__ double wsum[4];
@@ -214,6 +216,7 @@ template <class F, bool FIRST>
 __global__ void __launch_bounds__(128, F::id == 0 ? 3 : 8)
     k_adj_inv(Pops<const typename F::S> fp, Pops<const typename F::S> lin, Pops<typename F::S> lout,
               Pops<typename F::S> gout, int store_g, Geo g, typename F::R omega, typename F::R rinv, double* acc) {
+  step_begin();
   using S = typename F::S; using R = typename F::R;
   using D = R;
   __shared__ double wsum[4];
@@ -346,6 +349,7 @@ template <class F>
 __global__ void __launch_bounds__(DIAG_THREADS) k_tan_step(Pops<const typename F::S> f, Pops<const typename F::S> df,
                                                            Pops<typename F::S> f2, Pops<typename F::S> df2, Geo g,
                                                            typename F::R omega, typename F::R domega) {
+  step_begin();
   using S = typename F::S; using R = typename F::R; using V = typename F::V; using N = Num<V>;
   const long long n = (long long)g.nx * g.ny * g.nz;
   for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x) {
@@ -475,11 +479,15 @@ cudaError_t launch_adj_step(const Lattice& ft, const Lattice& lin, const Lattice
                             cudaStream_t st) {
   dim3 grid, block;
   adj_shape(ft.g, &grid, &block);
-  BGK_FORM_DISPATCH(ft,
-      (k_adj_step<F64><<<grid, block, 0, st>>>(pops<const double>(ft), pops<const double>(lin), pops<double>(lout),
-                                               ft.g, omega, acc)),
-      (k_adj_step<F32><<<grid, block, 0, st>>>(pops<const float>(ft), pops<const float>(lin), pops<float>(lout),
-                                               ft.g, (float)omega, acc)))
+  switch (ft.form) {
+    case FORM_F64:
+      return launch_step(k_adj_step<F64>, grid, block, st, pops<const double>(ft), pops<const double>(lin),
+                         pops<double>(lout), ft.g, omega, acc);
+    case FORM_F32:
+      return launch_step(k_adj_step<F32>, grid, block, st, pops<const float>(ft), pops<const float>(lin),
+                         pops<float>(lout), ft.g, (float)omega, acc);
+  }
+  return cudaErrorInvalidValue;
 }
 
 cudaError_t launch_adj_inv(const Lattice& post, bool first, const Lattice& lin, const Lattice& lout,
@@ -492,15 +500,13 @@ cudaError_t launch_adj_inv(const Lattice& post, bool first, const Lattice& lin, 
   switch (post.form) {
     case FORM_F64: {
       auto kf = first ? k_adj_inv<F64, true> : k_adj_inv<F64, false>;
-      kf<<<grid, block, 0, st>>>(pops<const double>(post), pops<const double>(lin), pops<double>(lout),
+      return launch_step(kf, grid, block, st, pops<const double>(post), pops<const double>(lin), pops<double>(lout),
                                  pops<double>(go), sg, post.g, omega, rinv, acc);
-      return cudaGetLastError();
     }
     case FORM_F32: {
       auto kf = first ? k_adj_inv<F32, true> : k_adj_inv<F32, false>;
-      kf<<<grid, block, 0, st>>>(pops<const float>(post), pops<const float>(lin), pops<float>(lout),
+      return launch_step(kf, grid, block, st, pops<const float>(post), pops<const float>(lin), pops<float>(lout),
                                  pops<float>(go), sg, post.g, (float)omega, (float)rinv, acc);
-      return cudaGetLastError();
     }
   }
   return cudaErrorInvalidValue;
@@ -525,13 +531,15 @@ cudaError_t launch_tan_init(const Lattice& df, const double* u0, const double* d
 
 cudaError_t launch_tan_step(const Lattice& f, const Lattice& df, const Lattice& f2, const Lattice& df2, double omega,
                             double domega, cudaStream_t st) {
-  BGK_FORM_DISPATCH(f,
-      (k_tan_step<F64><<<DIAG_BLOCKS, DIAG_THREADS, 0, st>>>(pops<const double>(f), pops<const double>(df),
-                                                             pops<double>(f2), pops<double>(df2), f.g, omega,
-                                                             domega)),
-      (k_tan_step<F32><<<DIAG_BLOCKS, DIAG_THREADS, 0, st>>>(pops<const float>(f), pops<const float>(df),
-                                                             pops<float>(f2), pops<float>(df2), f.g, (float)omega,
-                                                             (float)domega)))
+  switch (f.form) {
+    case FORM_F64:
+      return launch_step(k_tan_step<F64>, DIAG_BLOCKS, DIAG_THREADS, st, pops<const double>(f), pops<const double>(df),
+                         pops<double>(f2), pops<double>(df2), f.g, omega, domega);
+    case FORM_F32:
+      return launch_step(k_tan_step<F32>, DIAG_BLOCKS, DIAG_THREADS, st, pops<const float>(f), pops<const float>(df),
+                         pops<float>(f2), pops<float>(df2), f.g, (float)omega, (float)domega);
+  }
+  return cudaErrorInvalidValue;
 }
 
 cudaError_t launch_tan_loss(const Lattice& f, const Lattice& df, const double* ut, double* acc, cudaStream_t st) {

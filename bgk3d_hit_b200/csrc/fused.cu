@@ -33,6 +33,7 @@
 #include <cuda.h>
 
 #include "kernels.h"
+#include "launch.cuh"
 
 namespace bgk {
 
@@ -137,10 +138,8 @@ __global__ void __launch_bounds__(Two2<typename F::S, TY>::THREADS, 1)
   };
   auto next = [&](int p) { return p == g.nz - 1 ? 0 : p + 1; };
 
-  // a step after this one may be scheduled now; nothing of the step before is read
-  // or overwritten before it is done (step_begin of the single steps)
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  // nothing of the step before is read or overwritten before it is done
+  step_begin();
 
   if (tid == T::WORK) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&sm.bar[0])) : "memory");

@@ -24,6 +24,7 @@
 #include <cmath>
 
 #include "kernels.h"
+#include "launch.cuh"
 #include "reduce.cuh"
 #include "vec.cuh"
 
@@ -34,17 +35,6 @@ __device__ __forceinline__ int wrapi(int i, int n) { return i < 0 ? i + n : (i >
 __device__ __forceinline__ double ldg(const double* p) { return __ldg(p); }
 __device__ __forceinline__ float ldg(const float* p) { return __ldg(p); }
 __device__ __forceinline__ __half ldg(const __half* p) { return __ldg(p); }
-
-// Consecutive steps overlap their launches: a step's blocks are scheduled while the
-// last blocks of the step before still run (launch_step asks for it), and wait here
-// until all of that step's stores can be seen. First statement of every kernel
-// that launch_step launches. us per step without / with it on B200: FP64 32^3 4.1 /
-// 3.2, 64^3 10.7 / 9.0, 128^3 98.6 / 95.9; FP16 32^3 4.1 / 2.2, 64^3 6.2 / 4.9, 128^3
-// 28.7 / 26.0.
-__device__ __forceinline__ void step_begin() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-}
 
 // Moments of 19 local deviations in the reference's order
 // (SRC/diagno.F90:96-104, identical to SRC/col_MC.F90:133-141).
@@ -71,28 +61,6 @@ static Shape cell_shape(const Geo& g) {
   s.block = dim3(tx, ty, 1);
   s.grid = dim3((g.nx + tx - 1) / tx, (g.ny + ty - 1) / ty, g.nz);
   return s;
-}
-
-// Launches a kernel that starts with step_begin; overlap: so that it may be scheduled
-// beside the end of the kernel before it in the stream. Only on a context's own
-// stream, where that kernel is one of these or an ordinary one: step_begin waits
-// for the kernel before, and through its own for those before that.
-template <class... P, class... A>
-static cudaError_t launch_after(bool overlap, void (*kern)(P...), dim3 grid, dim3 block, cudaStream_t st, A... args) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.stream = st;
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &at;
-  cfg.numAttrs = overlap ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kern, P(args)...);
-}
-template <class... P, class... A>
-static cudaError_t launch_step(void (*kern)(P...), dim3 grid, dim3 block, cudaStream_t st, A... args) {
-  return launch_after(true, kern, grid, block, st, args...);
 }
 
 static int grid_1d(long long n, int threads, int cap) {
