@@ -41,7 +41,8 @@ namespace {
 
 constexpr int TX = 32;         // cells of a tile's row: one warp
 constexpr int PITCH = TX + 2;  // and of its first step, with the border
-constexpr int MAX_POLLS = 1 << 20;
+constexpr int MAX_POLLS = 1 << 16;  // of POLL_NS each at most: about a second
+constexpr int POLL_NS = 1 << 14;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -49,9 +50,9 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)_
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int polls) {
   for (int n = 0; n < polls; ++n) {
     uint32_t done;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n}\n"
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n}\n"
                  : "=r"(done)
-                 : "r"(bar), "r"(parity)
+                 : "r"(bar), "r"(parity), "r"(POLL_NS)
                  : "memory");
     if (done) return true;
   }
@@ -172,8 +173,12 @@ __global__ void __launch_bounds__(Two2<typename F::S, TY>::THREADS, 1)
   if (w == T::WORK / 32) {
     int z = next(next(modw(z0 - 1, g.nz)));
     for (int k = 0; k + 2 < np; ++k, z = next(z)) {
-      asm volatile("bar.sync 1, %0;" ::"n"(T::ATH + 32) : "memory");  // plane k has been read
+      // plane k has been read. Two barriers in turn: a warp comes to plane k + 2,
+      // which this warp asks for below, only after this wait is over, but may come
+      // to plane k + 1 before this warp comes here, and must not count for plane k
+      asm volatile("bar.sync %0, %1;" ::"r"(4 + (k & 1)), "n"(T::ATH + 32) : "memory");
       if (lane == 0) issue(k, z);
+      __syncwarp();
     }
   } else if (tid < T::ATH) {
     int r, c;  // first-step cell of this thread: row, column of the tile (-1 .. 32)
@@ -213,10 +218,11 @@ __global__ void __launch_bounds__(Two2<typename F::S, TY>::THREADS, 1)
     bool dead = false;
     for (int k = 0; k < np; ++k) {
       S* const raw = &sm.raw[k & 1][0][0];
-      if (!mbar_wait(smem_u32(&sm.bar[k & 1]), (k >> 1) & 1, dead ? 1 << 10 : MAX_POLLS)) {
+      if (!mbar_wait(smem_u32(&sm.bar[k & 1]), (k >> 1) & 1, dead ? 1 : MAX_POLLS)) {
         dead = true;  // reported; the remaining waits are short
         *err = 1;
       }
+      __syncwarp();
       if (yedge) {
 #pragma unroll
         for (int m = 0; m < T::NPE; ++m) {
@@ -231,7 +237,8 @@ __global__ void __launch_bounds__(Two2<typename F::S, TY>::THREADS, 1)
 #pragma unroll
         for (int q = 0; q < Q; ++q) v[q] = raw[q * T::RAW + (cxq(q) > 0 ? em : (cxq(q) < 0 ? ep : e0))];
       }
-      if (k + 2 < np) asm volatile("bar.arrive 1, %0;" ::"n"(T::ATH + 32) : "memory");
+      __syncwarp();
+      if (k + 2 < np) asm volatile("bar.arrive %0, %1;" ::"r"(4 + (k & 1)), "n"(T::ATH + 32) : "memory");
       if (on) {
         F::template cell<LES>(v, K);
         S* const b = sm.post[k & 1][0];
