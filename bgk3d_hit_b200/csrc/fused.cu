@@ -20,10 +20,10 @@
 // the periodic columns by a second, 32-byte wide box beside the first; rows beyond
 // a y face, which TMA fills with zeros, are put in by the threads.
 //
-// Measured on B200 at 256^3 FP64 (two steps): 992 us, 33.8 GLUPS, against 1515 us
-// (22.2, the HBM rate) for two single steps; DRAM 320 bytes a cell for both
-// (3.9 TB/s with the first layout), FP64 pipe about 55% busy. What stands between
-// it and the 37 GLUPS of its DRAM bytes is an interval of 2.0 us (collisions 1.1 us
+// Measured on B200 at 256^3 FP64 (two steps): 985 us, 34 GLUPS (1080-1110 us once the
+// power limit lowers the clock), against 1515 us (22.2, the HBM rate) for two single
+// steps; DRAM 305 bytes a cell for both, FP64 pipe 51% busy, issue slots 47%. What
+// stands between it and the 43 GLUPS of its DRAM bytes is the interval (1.1 us
 // of FP64 pipe, one barrier of all warps per plane). On the way there: both steps
 // by the same warps 25.6 GLUPS (too few warps between barriers), one raw buffer
 // 25.5 (the load of a plane did not fit beside its predecessor's collisions), loads
@@ -99,10 +99,17 @@ template <class S, int TY> struct Two2 {
 // time loop's lattices may lie elsewhere and has maps of its own.
 struct Two2Maps { CUtensorMap main, wrap, rest_main, rest_wrap; };
 
+// First plane of walk i: `full` walks of lz planes, then half of what is left at a
+// time, the last walk taking the rest.
+__device__ __forceinline__ int walk_begin(int i, int nz, int lz, int full) {
+  const int rest = nz - full * lz;
+  return i <= full ? i * lz : full * lz + rest - (rest >> (i - full));
+}
+
 template <class F, bool LES, int TY>
 __global__ void __launch_bounds__(Two2<typename F::S, TY>::THREADS, 1)
     k_two2(const __grid_constant__ Two2Maps maps, Pops<const typename F::S> src, Pops<typename F::S> dst, Geo g,
-           StepK K, int lz, int* err) {
+           StepK K, int lz, int full, int* err) {
   using S = typename F::S;
   using T = Two2<S, TY>;
   constexpr int ROWS = T::ROWS;
@@ -111,8 +118,10 @@ __global__ void __launch_bounds__(Two2<typename F::S, TY>::THREADS, 1)
   const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
   // the last tiles in y move down to end with the box: rows shared with their
   // neighbours are written twice, with the same bits
-  const int x0 = blockIdx.x * TX, y0 = min((int)blockIdx.y * TY, g.ny - TY), z0 = blockIdx.z * lz;
-  const int lzc = min(lz, g.nz - z0), txc = min(TX, g.nx - x0);
+  const int x0 = blockIdx.x * TX, y0 = min((int)blockIdx.y * TY, g.ny - TY);
+  const int z0 = walk_begin(blockIdx.z, g.nz, lz, full);
+  const int lzc = ((int)blockIdx.z + 1 < (int)gridDim.z ? walk_begin(blockIdx.z + 1, g.nz, lz, full) : g.nz) - z0;
+  const int txc = min(TX, g.nx - x0);
   const int plane = g.sx * g.ny;
   const int np = lzc + 2;                                    // first-step planes
   const bool left = x0 == 0, right = x0 + TX + 2 > g.nx;     // never both (nx >= 34)
@@ -360,8 +369,13 @@ cudaError_t launch(const Lattice& s, const Lattice& d, const StepK& K, cudaStrea
       !encode(&m.rest_main, g, s.form, s.p[Q - 1], 1, T::RP, T::ROWS) ||
       !encode(&m.rest_wrap, g, s.form, s.p[Q - 1], 1, T::WP, T::ROWS))
     return cudaErrorInvalidValue;
-  const int lz = best_walk(g, TY, SMS).lz;
-  const dim3 grid((g.nx + TX - 1) / TX, (g.ny + TY - 1) / TY, (g.nz + lz - 1) / lz);
+  // The last walk is halved twice, so that the SMs that are done first are not idle
+  // for a whole walk. Equal walks / halved, us per two steps of long runs: FP32 256^3
+  // 693 / 677, 180^3 271 / 265, 160^3 192 / 189; FP64 256^3 1136 / 1127, 128^3 174.9 /
+  // 173.6; Smagorinsky 256^3 1419 / 1418.
+  const int lz = best_walk(g, TY, SMS).lz, full = (g.nz + lz - 1) / lz - 1, rest = g.nz - full * lz;
+  const int halvings = rest >= 4 ? 2 : 0;
+  const dim3 grid((g.nx + TX - 1) / TX, (g.ny + TY - 1) / TY, full + 1 + halvings);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(T::THREADS);
@@ -372,7 +386,7 @@ cudaError_t launch(const Lattice& s, const Lattice& d, const StepK& K, cudaStrea
   at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, m, pops<const S>(s), pops<S>(d), g, K, lz, s.err);
+  return cudaLaunchKernelEx(&cfg, kern, m, pops<const S>(s), pops<S>(d), g, K, lz, full, s.err);
 }
 
 }  // namespace
