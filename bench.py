@@ -20,15 +20,15 @@ boundaries + col_MC). Prints one JSON line.
   tau = 0.502), initial field made on the GPU; max(K, 50) steps each, own
   clock record.
 - e2e: the same K steps through the public C-ABI as a user drives them: the
-  initial velocity field uploaded from pinned host memory, then
-  boundaries + col_MC + diagnostic every step (diagnostics computed every
+  initial velocity field uploaded from pinned host memory, then the time loop
+  (the steps between two diagnostics in one call, diagnostics computed every
   icheck = 100 steps, the reference's default, SRC/input.F90:221, and read
   back to the host), all inside the timed region, after an untimed warm-up
   pass of the same calls (upload, init and W steps); split into the one-time
   part (upload + init, fixed_ms) and the per-step part (per_step_ms).
 - roofline: algorithmic bytes of the stream-collide kernel (19 loads + 19
   stores per cell) per launch / average launch time, against the measured HBM
-  copy bandwidth.
+  copy bandwidth; steps_per_launch is 2 where a launch takes two steps.
 - cpu_baseline: the CPU oracle (C restatement of the reference's
   boundaries + col_MC, FP64, OpenMP over all host cores) on a bounded sample.
 - --impl reference: times that CPU implementation on this workload (rank 0),
@@ -306,14 +306,18 @@ def time_steps(box, steps, device):
     return ms, box.launch_count - l0, clocks.stop()
 
 
-def roofline_of(precision, scheme, L, ms_per_step, kernel=0, les=False):
+def roofline_of(precision, scheme, L, ms_per_step, kernel=0, les=False, launches_per_step=1.0):
+    """Bytes of the launches over their time: each moves every population of
+    every cell once in and once out, whether it takes one step or two."""
     bpc = BYTES_PER_CELL[precision]
     peak, peak_kind = measured_hbm()
-    achieved = bpc * float(L) ** 3 / (ms_per_step * 1e-3) / 1e9
+    achieved = bpc * float(L) ** 3 * launches_per_step / (ms_per_step * 1e-3) / 1e9
     kern = kernel_key(precision, scheme, L, kernel, les)
+    if launches_per_step < 1.0:  # two steps per launch (and a single one after an odd count)
+        kern = f"k_two2_{precision}" + ("_les" if les else "")
     tr = ncu_traffic(kern)
     return {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-            "traffic": tr * float(L) ** 3 if tr else None, "peak_kind": peak_kind, "bytes_per_cell": bpc,
+            "steps_per_launch": 1.0 / launches_per_step, "traffic": tr * float(L) ** 3 if tr else None, "peak_kind": peak_kind, "bytes_per_cell": bpc,
             "kernel": kern}
 
 
@@ -332,7 +336,7 @@ def form_line(a, precision, pin, device, fp64_value):
     finally:
         box.close()
     value = float(L) ** 3 * steps / (ms * 1e-3) / 1e9
-    rl = roofline_of(precision, "two_lattice", L, ms / steps)
+    rl = roofline_of(precision, "two_lattice", L, ms / steps, launches_per_step=launches / steps)
     if rl["traffic"] is not None:
         rl["traffic_note"] = "ncu DRAM bytes per cell of the 256^3 capture x cells"
     return {"value": value, "unit": "GLUPS", "ratio_vs_fp64": value / fp64_value, "steps": steps,
@@ -363,7 +367,7 @@ def large_line(a, L, precision, scheme, k0, tau, device):
     finally:
         box.close()
     value = float(L) ** 3 * steps / (ms * 1e-3) / 1e9
-    rl = roofline_of(precision, scheme, L, ms / steps)
+    rl = roofline_of(precision, scheme, L, ms / steps, launches_per_step=launches / steps)
     if rl["traffic"] is not None:
         rl["traffic_note"] = "ncu DRAM bytes per cell of the 256^3 capture x cells"
     noise = "numpy default_rng" if L ** 3 <= NUMPY_NOISE_MAX_CELLS else "torch CUDA generator"
@@ -430,7 +434,7 @@ def run_ours(a):
     ms_max = max_over_ranks(ms)
     lu = float(L) ** 3 * a.steps
     value = ws * lu / (ms_max * 1e-3) / 1e9
-    roofline = roofline_of(a.precision, a.scheme, L, ms / a.steps, a.kernel, a.les_cs > 0)
+    roofline = roofline_of(a.precision, a.scheme, L, ms / a.steps, a.kernel, a.les_cs > 0, launches / a.steps)
     box.close()
 
     # -------- e2e through the C-ABI with host buffers
@@ -444,9 +448,7 @@ def run_ours(a):
         # context's upload staging and the first-use costs of the pinned pages
         # stay out of the timed pass, which uploads and initialises again
         box2.init_velocity(*(p.numpy() for p in pin))
-        for it in range(1, a.warmup + 1):
-            box2.boundaries(it)
-            box2.col_MC(it)
+        box2.run(a.warmup)
         box2.synchronize()
         torch.cuda.synchronize()
         if ws > 1:
@@ -455,9 +457,11 @@ def run_ours(a):
         box2.init_velocity(*(p.numpy() for p in pin))
         evi.record(stream2)
         ndiag = 0
-        for it in range(1, a.steps + 1):
-            box2.boundaries(it)
-            box2.col_MC(it)
+        it = 0
+        while it < a.steps:  # the steps between two diagnostics in one call, as run_loop
+            n = min(a.steps - it, a.icheck - it % a.icheck)
+            box2.run(n)
+            it += n
             if box2.diagnostic(it) is not None or it == a.steps:
                 ndiag += 1
         if a.steps % a.icheck:
