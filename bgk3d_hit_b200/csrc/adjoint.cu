@@ -135,8 +135,8 @@ __global__ void __launch_bounds__(128, 4) k_adj_step(Pops<const typename F::S> f
     D L0 = 0, m1x = 0, m1y = 0, m1z = 0, mxx = 0, myy = 0, mzz = 0, mxy = 0, mxz = 0, myz = 0, S1 = 0;
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
-      const R x = (R)__ldg(ft.p[q] + offq(q, 1));
-      const D lam = (D)__ldg(lin.p[q] + offq(q, -1));
+      const R x = (R)ft.p[q][offq(q, 1)];
+      const D lam = (D)lin.p[q][offq(q, -1)];
       rho += x;
       jx += (R)cxq(q) * x;
       jy += (R)cyq(q) * x;
@@ -168,11 +168,13 @@ __global__ void __launch_bounds__(128, 4) k_adj_step(Pops<const typename F::S> f
     dw = (double)((D)rho * A - L0 - S1);
     const R om1 = (R)1 - omega;
     const R om = omega;
+    R lam[Q];  // all loads before the first store, behind which none of them may move
+#pragma unroll
+    for (int q = 0; q < Q; ++q) lam[q] = (R)lin.p[q][offq(q, -1)];
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
-      const R lam = (R)__ldg(lin.p[q] + offq(q, -1));
       const R gq = (R)(G + cdot<D>(q, Bx, By, Bz));
-      const R mu = om1 * lam + om * gq;
+      const R mu = om1 * lam[q] + om * gq;
       lout.p[q][o] = (S)mu;  // mu_q(x): cell x - c_q of the next adjoint step gathers it as its lam_q
     }
   }
@@ -209,14 +211,17 @@ __global__ void __launch_bounds__(128, 4) k_adj_step(Pops<const typename F::S> f
 // uses this only where |1 - omega|^-(K-1) is small over a segment of K steps.
 // Moment sums in the form's arithmetic, with fused multiply-adds, like
 // k_adj_step; the dL/domega term of each cell is added in double. Register
-// caps: 3 blocks/SM for FP64 (158 registers), 8 for FP32 (64); measured
+// caps: 3 blocks/SM for FP64 (164 registers), 8 for FP32 (64); measured
 // against 4 and 5 (FP64) and 4 and 6 (FP32), and against loading all 19
-// lam before the moment loop, all slower.
+// lam before the moment loop, all slower. Not overlapped with the launch before
+// (no step_begin), so that it may read by the read-only path: ordinary loads cannot
+// move over the stores of g, and with all stores behind all loads a step of the
+// gradient at 128^3 took 312.7 us instead of 301.2 (FP64) and 172.6 instead of
+// 167.5 (FP32), with the loads a few ahead of the stores 309-312 and 184-209.
 template <class F, bool FIRST>
 __global__ void __launch_bounds__(128, F::id == 0 ? 3 : 8)
     k_adj_inv(Pops<const typename F::S> fp, Pops<const typename F::S> lin, Pops<typename F::S> lout,
               Pops<typename F::S> gout, int store_g, Geo g, typename F::R omega, typename F::R rinv, double* acc) {
-  step_begin();
   using S = typename F::S; using R = typename F::R;
   using D = R;
   __shared__ double wsum[4];
@@ -500,13 +505,15 @@ cudaError_t launch_adj_inv(const Lattice& post, bool first, const Lattice& lin, 
   switch (post.form) {
     case FORM_F64: {
       auto kf = first ? k_adj_inv<F64, true> : k_adj_inv<F64, false>;
-      return launch_step(kf, grid, block, st, pops<const double>(post), pops<const double>(lin), pops<double>(lout),
+      kf<<<grid, block, 0, st>>>(pops<const double>(post), pops<const double>(lin), pops<double>(lout),
                                  pops<double>(go), sg, post.g, omega, rinv, acc);
+      return cudaGetLastError();
     }
     case FORM_F32: {
       auto kf = first ? k_adj_inv<F32, true> : k_adj_inv<F32, false>;
-      return launch_step(kf, grid, block, st, pops<const float>(post), pops<const float>(lin), pops<float>(lout),
+      kf<<<grid, block, 0, st>>>(pops<const float>(post), pops<const float>(lin), pops<float>(lout),
                                  pops<float>(go), sg, post.g, (float)omega, (float)rinv, acc);
+      return cudaGetLastError();
     }
   }
   return cudaErrorInvalidValue;

@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(Two2<typename F::S, TY>::THREADS, 1)
         const int e = tid + m * T::ATH, n = e / T::YCOLS;
         if (n < yn) {
           const int q = sm.yrq[n] >> 6, cz = czq(q);
-          yv[m] = __ldg(sm.base[q] + (sm.yrow[n] + modw(x0 + e % T::YCOLS - 2, g.nx) + (cz > 0 ? zm : (cz < 0 ? zp : zc))));
+          yv[m] = sm.base[q][sm.yrow[n] + modw(x0 + e % T::YCOLS - 2, g.nx) + (cz > 0 ? zm : (cz < 0 ? zp : zc))];
         }
       }
       zy = next(zy);

@@ -32,6 +32,7 @@ namespace bgk {
 
 __device__ __forceinline__ int wrapi(int i, int n) { return i < 0 ? i + n : (i >= n ? i - n : i); }
 
+// Read-only loads, for the kernels that no launch overlaps (see step_begin).
 __device__ __forceinline__ double ldg(const double* p) { return __ldg(p); }
 __device__ __forceinline__ float ldg(const float* p) { return __ldg(p); }
 __device__ __forceinline__ __half ldg(const __half* p) { return __ldg(p); }
@@ -91,9 +92,9 @@ __global__ void __launch_bounds__(256) k_two(Pops<const typename F::S> src, Pops
     const int jj = cyq(q) > 0 ? jm : (cyq(q) < 0 ? jp : j);
     const int kk = czq(q) > 0 ? km : (czq(q) < 0 ? kp : k);
     const int off = ii + g.sx * (jj + g.ny * kk);
-    // pop 19 with a plain load: in the time loop it is updated in place
-    // (src.p[18] == dst.p[18]); the adjoint's out-of-place steps pass distinct arrays
-    v[q] = (q == Q - 1) ? src.p[Q - 1][off] : ldg(src.p[q] + off);
+    // pop 19: in the time loop it is updated in place (src.p[18] == dst.p[18]); the
+    // adjoint's out-of-place steps pass distinct arrays
+    v[q] = src.p[q][off];
   }
   F::template cell<LES>(v, K);
   const int o = i + g.sx * (j + g.ny * k);
@@ -132,10 +133,10 @@ __global__ void __launch_bounds__(128, 5) k_two_f16v(Pops<const __half> src, Pop
     const int jj = cyq(q) > 0 ? jm : (cyq(q) < 0 ? jp : j);
     const int kk = czq(q) > 0 ? km : (czq(q) < 0 ? kp : k);
     const __half* p = (q == Q - 1 ? (const __half*)dst.p[Q - 1] : src.p[q]) + g.sx * (jj + g.ny * kk);
-    Y[q] = (q == Q - 1) ? *reinterpret_cast<const uint2*>(p + i0) : __ldg(reinterpret_cast<const uint2*>(p + i0));
+    Y[q] = *reinterpret_cast<const uint2*>(p + i0);
     E[q] = 0;
-    if (cxq(q) > 0 && xl.edge_prev) E[q] = ldg_u16(p + at.i_prev);
-    if (cxq(q) < 0 && xl.edge_next) E[q] = ldg_u16(p + at.i_next);
+    if (cxq(q) > 0 && xl.edge_prev) E[q] = u16_at(p + at.i_prev);
+    if (cxq(q) < 0 && xl.edge_next) E[q] = u16_at(p + at.i_next);
   }
   if (at.last()) wrap_last(Y, E, at.cells);
   shift_rows(Y, E, xl);
@@ -167,13 +168,12 @@ __global__ void __launch_bounds__(128, 5) k_two_f32v(Pops<const float> src, Pops
   for (int q = 0; q < Q; ++q) {
     const int jj = cyq(q) > 0 ? jm : (cyq(q) < 0 ? jp : j);
     const int kk = czq(q) > 0 ? km : (czq(q) < 0 ? kp : k);
-    // pop 19 with a plain load: in the time loop it is updated in place
-    // (src.p[18] == dst.p[18]); the adjoint's out-of-place steps pass distinct arrays
+    // pop 19: updated in place in the time loop, distinct arrays in the adjoint's steps
     const float* p = src.p[q] + g.sx * (jj + g.ny * kk);
-    Y[q] = (q == Q - 1) ? *reinterpret_cast<const float2*>(p + i0) : __ldg(reinterpret_cast<const float2*>(p + i0));
+    Y[q] = *reinterpret_cast<const float2*>(p + i0);
     E[q] = 0.f;
-    if (cxq(q) > 0 && xl.edge_prev) E[q] = __ldg(p + at.i_prev);
-    if (cxq(q) < 0 && xl.edge_next) E[q] = __ldg(p + at.i_next);
+    if (cxq(q) > 0 && xl.edge_prev) E[q] = *(p + at.i_prev);
+    if (cxq(q) < 0 && xl.edge_next) E[q] = *(p + at.i_next);
   }
   if (at.last()) wrap_last(Y, E, at.cells);
   shift_rows_f32(Y, E, xl);
@@ -227,17 +227,16 @@ __global__ void __launch_bounds__(256, 4) k_two_f16v2(Pops<const __half> src, Po
     const int jj = cyq(q) > 0 ? jm : (cyq(q) < 0 ? jp : j);
     const int kk = czq(q) > 0 ? km : (czq(q) < 0 ? kp : k);
     const __half* p = (q == Q - 1 ? (const __half*)dst.p[Q - 1] : src.p[q]) + g.sx * (jj + g.ny * kk);
-    const unsigned A = (q == Q - 1) ? *reinterpret_cast<const unsigned*>(p + i0)
-                                    : __ldg(reinterpret_cast<const unsigned*>(p + i0));
+    const unsigned A = *reinterpret_cast<const unsigned*>(p + i0);
     if (cxq(q) == 0) {
       Y[q] = A;
     } else if (cxq(q) > 0) {  // cells need elements i0-1, i0
       unsigned prev = __shfl_sync(0xffffffffu, A >> 16, src_prev);
-      if (load_prev) prev = ldg_u16(p + i_prev);
+      if (load_prev) prev = u16_at(p + i_prev);
       Y[q] = __byte_perm(A, prev, 0x1054);
     } else {  // cells need elements i0+1, i0+2
       unsigned next = __shfl_sync(0xffffffffu, A & 0xffffu, src_next);
-      if (load_next) next = ldg_u16(p + i_next);
+      if (load_next) next = u16_at(p + i_next);
       Y[q] = __byte_perm(A, next, 0x5432);
     }
   }
@@ -274,30 +273,30 @@ __global__ void __launch_bounds__(256, 4) k_two_f16v2(Pops<const __half> src, Po
 // Even step: g_q(x) = slot q at x; result q -> slot opp(q) at x.
 // Odd step:  g_q(x) = slot opp(q) at x - c_q; result q -> slot q at x + c_q.
 // Each thread reads exactly the locations it writes, so the update is
-// race-free in place; a location is never read after it has been written,
-// which also makes the read-only load path safe.
+// race-free in place; a location is never read after it has been written.
 template <class F, bool ODD, bool LES>
 __device__ __forceinline__ void aa_cell(Pops<typename F::S>& a, const Geo& g, const StepK& K) {
   using S = typename F::S;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y;
-  const int k = blockIdx.z;
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  int j = blockIdx.y * blockDim.y + threadIdx.y;
+  int k = blockIdx.z;
   if (i >= g.nx || j >= g.ny) return;
-  const int o = i + g.sx * (j + g.ny * k);
-  const int im = i == 0 ? g.nx - 1 : i - 1, ip = i == g.nx - 1 ? 0 : i + 1;
-  const int jm = j == 0 ? g.ny - 1 : j - 1, jp = j == g.ny - 1 ? 0 : j + 1;
-  const int km = k == 0 ? g.nz - 1 : k - 1, kp = k == g.nz - 1 ? 0 : k + 1;
+  int o = i + g.sx * (j + g.ny * k);
   // location x - c_q (read, slot opp(q)) == location x + c_opp(q) (write, slot opp(q))
   auto back = [&](int q) {
-    const int ii = cxq(q) > 0 ? im : (cxq(q) < 0 ? ip : i);
-    const int jj = cyq(q) > 0 ? jm : (cyq(q) < 0 ? jp : j);
-    const int kk = czq(q) > 0 ? km : (czq(q) < 0 ? kp : k);
+    const int ii = cxq(q) > 0 ? (i == 0 ? g.nx - 1 : i - 1) : (cxq(q) < 0 ? (i == g.nx - 1 ? 0 : i + 1) : i);
+    const int jj = cyq(q) > 0 ? (j == 0 ? g.ny - 1 : j - 1) : (cyq(q) < 0 ? (j == g.ny - 1 ? 0 : j + 1) : j);
+    const int kk = czq(q) > 0 ? (k == 0 ? g.nz - 1 : k - 1) : (czq(q) < 0 ? (k == g.nz - 1 ? 0 : k + 1) : k);
     return ii + g.sx * (jj + g.ny * kk);
   };
   S v[Q];
 #pragma unroll
-  for (int q = 0; q < Q; ++q) v[q] = ODD ? ldg(a.p[oppq(q)] + back(q)) : ldg(a.p[q] + o);
+  for (int q = 0; q < Q; ++q) v[q] = ODD ? a.p[oppq(q)][back(q)] : a.p[q][o];
   F::template cell<LES>(v, K);
+  // the stores go to the places of the loads: recomputed, or the compiler keeps all
+  // addresses through the collision (FP64 even step 124 registers instead of 80)
+  if (ODD) asm volatile("" : "+r"(i), "+r"(j), "+r"(k));
+  else asm volatile("" : "+r"(o));
 #pragma unroll
   for (int q = 0; q < Q; ++q) {
     if (ODD) a.p[q][back(oppq(q))] = v[q];
@@ -419,16 +418,16 @@ __global__ void __launch_bounds__(128, 5) k_aa_f16v(Pops<__half> a, Geo g, StepK
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
       const __half* p = a.p[oppq(q)] + row(-cyq(q), -czq(q));
-      Y[q] = __ldg(reinterpret_cast<const uint2*>(p + i0));
+      Y[q] = *reinterpret_cast<const uint2*>(p + i0);
       E[q] = 0;
-      if (cxq(q) > 0 && xl.edge_prev) E[q] = ldg_u16(p + at.i_prev);
-      if (cxq(q) < 0 && xl.edge_next) E[q] = ldg_u16(p + at.i_next);
+      if (cxq(q) > 0 && xl.edge_prev) E[q] = u16_at(p + at.i_prev);
+      if (cxq(q) < 0 && xl.edge_next) E[q] = u16_at(p + at.i_next);
     }
     if (at.last()) wrap_last(Y, E, at.cells);
     shift_rows(Y, E, xl);
   } else {
 #pragma unroll
-    for (int q = 0; q < Q; ++q) Y[q] = __ldg(reinterpret_cast<const uint2*>(a.p[q] + row(0, 0) + i0));
+    for (int q = 0; q < Q; ++q) Y[q] = *reinterpret_cast<const uint2*>(a.p[q] + row(0, 0) + i0);
   }
   if (FLAT || valid) collide4_f16<LES>(Y, K);
   // odd step: the warps' crossing values (cx > 0 populations: the last
@@ -456,7 +455,7 @@ __global__ void __launch_bounds__(128, 5) k_aa_f16v(Pops<__half> a, Geo g, StepK
   const XLanes xs = FLAT ? XLanes(as, threadIdx.x & 31) : xl;
   const EdgeWarps es = FLAT ? EdgeWarps(as) : ew;
   int js = FLAT ? as.j : j, ks = k;  // store rows: recomputed after the collision (BGK odd step)
-  if (ODD) asm volatile("" : "+r"(js), "+r"(ks));
+  asm volatile("" : "+r"(js), "+r"(ks));
   const int jms = js == 0 ? g.ny - 1 : js - 1, jps = js == g.ny - 1 ? 0 : js + 1;
   const int kms = ks == 0 ? g.nz - 1 : ks - 1, kps = ks == g.nz - 1 ? 0 : ks + 1;
   auto row_out = [&](int dy, int dz) {
@@ -467,7 +466,7 @@ __global__ void __launch_bounds__(128, 5) k_aa_f16v(Pops<__half> a, Geo g, StepK
 #pragma unroll
   for (int q = 0; q < Q; ++q) {
     if (!ODD) {
-      *reinterpret_cast<uint2*>(a.p[oppq(q)] + row(0, 0) + i0) = Y[q];
+      *reinterpret_cast<uint2*>(a.p[oppq(q)] + row_out(0, 0) + i0) = Y[q];
     } else {
       const unsigned fp = cxq(q) > 0 && xs.edge_prev && es.prev_in ? xs_last[es.wprev][q] : 0u;
       const unsigned fn = cxq(q) < 0 && xs.edge_next && es.next_in ? xs_first[es.wnext][q - 9] : 0u;
@@ -571,15 +570,15 @@ __global__ void __launch_bounds__(128, 4) k_aa_f16w(Pops<__half> a, Geo g, StepK
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
       const __half* p = a.p[oppq(q)] + row(-cyq(q), -czq(q));
-      Y[q] = __ldg(reinterpret_cast<const uint4*>(p + i0));
+      Y[q] = *reinterpret_cast<const uint4*>(p + i0);
       E[q] = 0;
-      if (cxq(q) > 0 && xl.edge_prev) E[q] = ldg_u16(p + at.i_prev);
-      if (cxq(q) < 0 && xl.edge_next) E[q] = ldg_u16(p + at.i_next);
+      if (cxq(q) > 0 && xl.edge_prev) E[q] = u16_at(p + at.i_prev);
+      if (cxq(q) < 0 && xl.edge_next) E[q] = u16_at(p + at.i_next);
     }
     shift_rows8(Y, E, xl);
   } else {
 #pragma unroll
-    for (int q = 0; q < Q; ++q) Y[q] = __ldg(reinterpret_cast<const uint4*>(a.p[q] + row(0, 0) + i0));
+    for (int q = 0; q < Q; ++q) Y[q] = *reinterpret_cast<const uint4*>(a.p[q] + row(0, 0) + i0);
   }
   if (FLAT || valid) {
     uint2 L[Q], H[Q];
@@ -614,7 +613,7 @@ __global__ void __launch_bounds__(128, 4) k_aa_f16w(Pops<__half> a, Geo g, StepK
   const XLanes xs = FLAT ? XLanes(as, threadIdx.x & 31) : xl;
   const EdgeWarps es = FLAT ? EdgeWarps(as) : ew;
   int js = FLAT ? as.j : j, ks = k;
-  if (ODD) asm volatile("" : "+r"(js), "+r"(ks));
+  asm volatile("" : "+r"(js), "+r"(ks));
   const int jms = js == 0 ? g.ny - 1 : js - 1, jps = js == g.ny - 1 ? 0 : js + 1;
   const int kms = ks == 0 ? g.nz - 1 : ks - 1, kps = ks == g.nz - 1 ? 0 : ks + 1;
   auto row_out = [&](int dy, int dz) {
@@ -625,7 +624,7 @@ __global__ void __launch_bounds__(128, 4) k_aa_f16w(Pops<__half> a, Geo g, StepK
 #pragma unroll
   for (int q = 0; q < Q; ++q) {
     if (!ODD) {
-      *reinterpret_cast<uint4*>(a.p[oppq(q)] + row(0, 0) + i0) = Y[q];
+      *reinterpret_cast<uint4*>(a.p[oppq(q)] + row_out(0, 0) + i0) = Y[q];
     } else {
       const unsigned fp = cxq(q) > 0 && xs.edge_prev && es.prev_in ? xs_last[es.wprev][q] : 0u;
       const unsigned fn = cxq(q) < 0 && xs.edge_next && es.next_in ? xs_first[es.wnext][q - 9] : 0u;
@@ -690,16 +689,16 @@ __global__ void __launch_bounds__(128, 5) k_aa_f32v(Pops<float> a, Geo g, StepK 
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
       const float* p = a.p[oppq(q)] + row(-cyq(q), -czq(q));
-      Y[q] = __ldg(reinterpret_cast<const float2*>(p + i0));
+      Y[q] = *reinterpret_cast<const float2*>(p + i0);
       E[q] = 0.f;
-      if (cxq(q) > 0 && xl.edge_prev) E[q] = __ldg(p + at.i_prev);
-      if (cxq(q) < 0 && xl.edge_next) E[q] = __ldg(p + at.i_next);
+      if (cxq(q) > 0 && xl.edge_prev) E[q] = *(p + at.i_prev);
+      if (cxq(q) < 0 && xl.edge_next) E[q] = *(p + at.i_next);
     }
     if (at.last()) wrap_last(Y, E, at.cells);
     shift_rows_f32(Y, E, xl);
   } else {
 #pragma unroll
-    for (int q = 0; q < Q; ++q) Y[q] = __ldg(reinterpret_cast<const float2*>(a.p[q] + row(0, 0) + i0));
+    for (int q = 0; q < Q; ++q) Y[q] = *reinterpret_cast<const float2*>(a.p[q] + row(0, 0) + i0);
   }
   if (FLAT || valid) {
 #pragma unroll
@@ -733,7 +732,7 @@ __global__ void __launch_bounds__(128, 5) k_aa_f32v(Pops<float> a, Geo g, StepK 
     if (!valid) return;
   }
   int js = j, ks = k;  // store rows: recomputed after the collision
-  if (ODD) asm volatile("" : "+r"(js), "+r"(ks));
+  asm volatile("" : "+r"(js), "+r"(ks));
   const int jms = js == 0 ? g.ny - 1 : js - 1, jps = js == g.ny - 1 ? 0 : js + 1;
   const int kms = ks == 0 ? g.nz - 1 : ks - 1, kps = ks == g.nz - 1 ? 0 : ks + 1;
   auto row_out = [&](int dy, int dz) {
@@ -744,7 +743,7 @@ __global__ void __launch_bounds__(128, 5) k_aa_f32v(Pops<float> a, Geo g, StepK 
 #pragma unroll
   for (int q = 0; q < Q; ++q) {
     if (!ODD) {
-      *reinterpret_cast<float2*>(a.p[oppq(q)] + row(0, 0) + i0) = Y[q];
+      *reinterpret_cast<float2*>(a.p[oppq(q)] + row_out(0, 0) + i0) = Y[q];
     } else {
       const float fp = cxq(q) > 0 && xl.edge_prev && ew.prev_in ? xs_last[ew.wprev][q] : 0.f;
       const float fn = cxq(q) < 0 && xl.edge_next && ew.next_in ? xs_first[ew.wnext][q - 9] : 0.f;
@@ -812,10 +811,10 @@ __global__ void __launch_bounds__(128, 4) k_aa_f32w(Pops<float> a, Geo g, StepK 
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
       const float* p = a.p[oppq(q)] + row(-cyq(q), -czq(q));
-      Y[q] = __ldg(reinterpret_cast<const float4*>(p + i0));
+      Y[q] = *reinterpret_cast<const float4*>(p + i0);
       E[q] = 0.f;
-      if (cxq(q) > 0 && xl.edge_prev) E[q] = __ldg(p + at.i_prev);
-      if (cxq(q) < 0 && xl.edge_next) E[q] = __ldg(p + at.i_next);
+      if (cxq(q) > 0 && xl.edge_prev) E[q] = *(p + at.i_prev);
+      if (cxq(q) < 0 && xl.edge_next) E[q] = *(p + at.i_next);
     }
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
@@ -1239,7 +1238,7 @@ static int diag_blocks(int form) { return 148 * diag_blocks_per_sm(form); }
 template <class F, int LAY, int PULL>
 __global__ void __launch_bounds__(DIAG_THREADS, diag_blocks_per_sm(F::id))
     k_diag(Pops<const typename F::S> a, Geo g, double svisc, double omega, typename F::R inv, double* partials,
-           typename F::R* vel, Halo<typename F::S> h, const typename F::S* __restrict__ faith, int faith_zero) {
+           typename F::R* vel, Halo<typename F::S> h, const typename F::S* faith, int faith_zero) {
   step_begin();
   using R = typename F::R; using V = typename F::V; using N = Num<V>;
   __shared__ KS sh[DIAG_THREADS / 32][NDK];
@@ -1260,7 +1259,7 @@ __global__ void __launch_bounds__(DIAG_THREADS, diag_blocks_per_sm(F::id))
     V x[Q];
 #pragma unroll
     for (int q = 0; q < Q; ++q)
-      x[q] = N::wrap(F::dec(ldg(a.p[ref_slot<LAY>(q)] + around_off<LAY, false>(nb, q)), inv));
+      x[q] = N::wrap(F::dec(a.p[ref_slot<LAY>(q)][around_off<LAY, false>(nb, q)], inv));
     V ux, uy, uz;
     const V rho = moments<V>(x, ux, uy, uz);
     const V ke = N::c(0.5) * (ux * ux + uy * uy + uz * uz);
@@ -1270,12 +1269,6 @@ __global__ void __launch_bounds__(DIAG_THREADS, diag_blocks_per_sm(F::id))
     kadd(acc[3], (double)N::raw(uz));
     kadd(acc[4], (double)N::raw(ke));
     if (!isfinite(N::raw(rho)) || !isfinite(N::raw(ux)) || !isfinite(N::raw(uy)) || !isfinite(N::raw(uz))) ++bad;
-    if (vel) {
-      const long long c = i + (long long)g.nx * (j + (long long)g.ny * k);
-      vel[c] = N::raw(ux);
-      vel[n + c] = N::raw(uy);
-      vel[2 * n + c] = N::raw(uz);
-    }
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
       const int si = i - cxq(q), sj = j - cyq(q), sk = k - czq(q);
@@ -1289,8 +1282,14 @@ __global__ void __launch_bounds__(DIAG_THREADS, diag_blocks_per_sm(F::id))
         const long long per = 2 * ((long long)g.ny * g.nz + (long long)g.nx * g.nz + (long long)g.nx * g.ny);
         x[q] = faith_zero ? N::c(0.0) : N::wrap(F::dec(faith[q * per + faith_off(g, si, sj, sk)], inv));
       } else {
-        x[q] = N::wrap(F::dec(ldg(a.p[ref_slot<LAY>(q)] + around_off<LAY, true>(nb, q)), inv));
+        x[q] = N::wrap(F::dec(a.p[ref_slot<LAY>(q)][around_off<LAY, true>(nb, q)], inv));
       }
+    }
+    if (vel) {  // behind the pulls: none of these loads may move over a store
+      const long long c = i + (long long)g.nx * (j + (long long)g.ny * k);
+      vel[c] = N::raw(ux);
+      vel[n + c] = N::raw(uy);
+      vel[2 * n + c] = N::raw(uz);
     }
     V e[Q], vx, vy, vz;
     const V rp = equilibrium<V>(x, e, vx, vy, vz);
@@ -1338,7 +1337,7 @@ __global__ void __launch_bounds__(256) k_velocity(Pops<const typename F::S> a, G
 }
 
 template <class R>
-__global__ void __launch_bounds__(DIAG_THREADS) k_enstrophy(const R* __restrict__ vel, int nx, int ny, int nz,
+__global__ void __launch_bounds__(DIAG_THREADS) k_enstrophy(const R* vel, int nx, int ny, int nz,
                                                            double* partials) {
   step_begin();
   __shared__ KS sh[DIAG_THREADS / 32][1];
@@ -1360,7 +1359,7 @@ __global__ void __launch_bounds__(DIAG_THREADS) k_enstrophy(const R* __restrict_
     const R* const rkp = vel + (long long)nx * (j + (long long)ny * kp);
     const R* const rkm = vel + (long long)nx * (j + (long long)ny * km);
     using E = Ex<double>;
-    auto D = [&](const R* p, int s, const R* m, int t) -> E { return E{0.5} * (E{(double)__ldg(p + s)} - E{(double)__ldg(m + t)}); };
+    auto D = [&](const R* p, int s, const R* m, int t) -> E { return E{0.5} * (E{(double)p[s]} - E{(double)m[t]}); };
     const E dwdy = D(rjp + 2 * n, i, rjm + 2 * n, i), dvdz = D(rkp + n, i, rkm + n, i);
     const E dudz = D(rkp, i, rkm, i), dwdx = D(row + 2 * n, ip, row + 2 * n, im);
     const E dvdx = D(row + n, ip, row + n, im), dudy = D(rjp, i, rjm, i);
@@ -1377,7 +1376,7 @@ __global__ void __launch_bounds__(DIAG_THREADS) k_enstrophy(const R* __restrict_
 // One block per quantity (one block for all ten took 16 us). totals may be
 // pinned host memory; err (optional): the device's error flag, copied behind
 // the ND + 1 totals so that the host reads one place.
-__global__ void __launch_bounds__(DIAG_THREADS) k_finalize(const double* __restrict__ partials, int blocks,
+__global__ void __launch_bounds__(DIAG_THREADS) k_finalize(const double* partials, int blocks,
                                                            double* totals, const int* err) {
   step_begin();
   __shared__ KS sh[DIAG_THREADS / 32][1];
@@ -1385,7 +1384,7 @@ __global__ void __launch_bounds__(DIAG_THREADS) k_finalize(const double* __restr
   KS acc[1] = {{0.0, 0.0}};
   const int nb = d < NDK ? blocks : DIAG_BLOCKS;  // k_diag's, k_enstrophy's
   for (int b = threadIdx.x; b < nb; b += blockDim.x) {
-    const double2 p = __ldg(reinterpret_cast<const double2*>(partials) + b * ND + d);
+    const double2 p = reinterpret_cast<const double2*>(partials)[b * ND + d];
     kcomb(acc[0], KS{p.x, p.y});
   }
   const KS r = block_reduce_n<1, DIAG_THREADS>(acc, sh);

@@ -10,6 +10,11 @@ namespace bgk {
 // that launch_step launches. us per step without / with it on B200: FP64 32^3 4.1 /
 // 3.2, 64^3 10.7 / 9.0, 128^3 98.6 / 95.9; FP16 32^3 4.1 / 2.2, 64^3 6.2 / 4.9, 128^3
 // 28.7 / 26.0.
+//
+// Everything behind it is read with ordinary loads: no __ldg, no const __restrict__
+// parameter. Its blocks are resident while the kernel before still writes, and
+// ld.global.nc is defined only for data that nothing writes as long as the kernel
+// that reads it runs; the wait above orders ordinary accesses and no others.
 __device__ __forceinline__ void step_begin() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");

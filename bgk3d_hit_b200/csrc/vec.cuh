@@ -6,9 +6,7 @@
 
 namespace bgk {
 
-__device__ __forceinline__ unsigned short ldg_u16(const __half* p) {
-  return __ldg(reinterpret_cast<const unsigned short*>(p));
-}
+__device__ __forceinline__ unsigned short u16_at(const __half* p) { return *reinterpret_cast<const unsigned short*>(p); }
 __device__ __forceinline__ unsigned h2u(__half2 h) { return *reinterpret_cast<unsigned*>(&h); }
 __device__ __forceinline__ float2 u2f2(unsigned u) { return __half22float2(*reinterpret_cast<__half2*>(&u)); }
 
