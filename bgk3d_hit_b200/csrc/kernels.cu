@@ -293,10 +293,13 @@ __device__ __forceinline__ void aa_cell(Pops<typename F::S>& a, const Geo& g, co
 #pragma unroll
   for (int q = 0; q < Q; ++q) v[q] = ODD ? a.p[oppq(q)][back(q)] : a.p[q][o];
   F::template cell<LES>(v, K);
-  // the stores go to the places of the loads: recomputed, or the compiler keeps all
-  // addresses through the collision (FP64 even step 124 registers instead of 80)
-  if (ODD) asm volatile("" : "+r"(i), "+r"(j), "+r"(k));
-  else asm volatile("" : "+r"(o));
+  // The stores go to the places of the loads. Left alone, the compiler keeps all their
+  // addresses through the collision (even step, FP64: 124 registers instead of 80).
+  // Recomputed in the odd step of FP16 and of the Smagorinsky collision only; GLUPS of
+  // the pair of steps at 256^3, recomputed / kept: FP16 62 / 51, Smagorinsky FP64 19.2 /
+  // 15.8, FP32 38.5 / 35.4, but FP64 19.6 / 21.6, FP32 39.2 / 40.1.
+  if (ODD && (LES || F::id == FORM_F16)) asm volatile("" : "+r"(i), "+r"(j), "+r"(k));
+  if (!ODD) asm volatile("" : "+r"(o));
 #pragma unroll
   for (int q = 0; q < Q; ++q) {
     if (ODD) a.p[q][back(oppq(q))] = v[q];
