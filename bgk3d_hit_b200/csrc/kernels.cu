@@ -277,32 +277,38 @@ __global__ void __launch_bounds__(256, 4) k_two_f16v2(Pops<const __half> src, Po
 template <class F, bool ODD, bool LES>
 __device__ __forceinline__ void aa_cell(Pops<typename F::S>& a, const Geo& g, const StepK& K) {
   using S = typename F::S;
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  int j = blockIdx.y * blockDim.y + threadIdx.y;
-  int k = blockIdx.z;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = blockIdx.y * blockDim.y + threadIdx.y;
+  const int k = blockIdx.z;
   if (i >= g.nx || j >= g.ny) return;
   int o = i + g.sx * (j + g.ny * k);
-  // location x - c_q (read, slot opp(q)) == location x + c_opp(q) (write, slot opp(q))
-  auto back = [&](int q) {
-    const int ii = cxq(q) > 0 ? (i == 0 ? g.nx - 1 : i - 1) : (cxq(q) < 0 ? (i == g.nx - 1 ? 0 : i + 1) : i);
-    const int jj = cyq(q) > 0 ? (j == 0 ? g.ny - 1 : j - 1) : (cyq(q) < 0 ? (j == g.ny - 1 ? 0 : j + 1) : j);
-    const int kk = czq(q) > 0 ? (k == 0 ? g.nz - 1 : k - 1) : (czq(q) < 0 ? (k == g.nz - 1 ? 0 : k + 1) : k);
-    return ii + g.sx * (jj + g.ny * kk);
-  };
+  const int im = i == 0 ? g.nx - 1 : i - 1, ip = i == g.nx - 1 ? 0 : i + 1;
+  const int jm = j == 0 ? g.ny - 1 : j - 1, jp = j == g.ny - 1 ? 0 : j + 1;
+  const int km = k == 0 ? g.nz - 1 : k - 1, kp = k == g.nz - 1 ? 0 : k + 1;
   S v[Q];
-#pragma unroll
-  for (int q = 0; q < Q; ++q) v[q] = ODD ? a.p[oppq(q)][back(q)] : a.p[q][o];
-  F::template cell<LES>(v, K);
-  // The stores go to the places of the loads. Left alone, the compiler keeps all their
-  // addresses through the collision (even step, FP64: 124 registers instead of 80).
-  // Recomputed in the odd step of FP16 and of the Smagorinsky collision only; GLUPS of
-  // the pair of steps at 256^3, recomputed / kept: FP16 62 / 51, Smagorinsky FP64 19.2 /
-  // 15.8, FP32 38.5 / 35.4, but FP64 19.6 / 21.6, FP32 39.2 / 40.1.
-  if (ODD && (LES || F::id == FORM_F16)) asm volatile("" : "+r"(i), "+r"(j), "+r"(k));
-  if (!ODD) asm volatile("" : "+r"(o));
+  int off[Q];  // location x - c_q (read, slot opp(q)) == location x + c_opp(q) (write, slot opp(q))
 #pragma unroll
   for (int q = 0; q < Q; ++q) {
-    if (ODD) a.p[q][back(oppq(q))] = v[q];
+    const int ii = cxq(q) > 0 ? im : (cxq(q) < 0 ? ip : i);
+    const int jj = cyq(q) > 0 ? jm : (cyq(q) < 0 ? jp : j);
+    const int kk = czq(q) > 0 ? km : (czq(q) < 0 ? kp : k);
+    off[q] = ii + g.sx * (jj + g.ny * kk);
+    v[q] = ODD ? a.p[oppq(q)][off[q]] : a.p[q][o];
+  }
+  F::template cell<LES>(v, K);
+  // The stores go to the places of the loads. The offsets are kept through the
+  // collision, not the 64-bit addresses, which the compiler would hold otherwise
+  // (FP64 124 registers, Smagorinsky 136). GLUPS of the pair of steps at 256^3, addresses
+  // kept / offsets recomputed / offsets kept: FP64 21.6 / 19.6 / 21.9, Smagorinsky 15.8 /
+  // 19.6 / 20.9; FP32 40.1 / 39.2 / 41.5, Smagorinsky 35.4 / 40.5 / 38.3; FP16 51 / 62 /
+  // 61.5, Smagorinsky 55 / 56.5 / 59.
+  if (!ODD) asm volatile("" : "+r"(o));
+#pragma unroll
+  for (int q = 0; q < Q; ++q)
+    if (ODD) asm volatile("" : "+r"(off[q]));
+#pragma unroll
+  for (int q = 0; q < Q; ++q) {
+    if (ODD) a.p[q][off[oppq(q)]] = v[q];
     else a.p[oppq(q)][o] = v[q];
   }
 }
@@ -457,7 +463,7 @@ __global__ void __launch_bounds__(128, 5) k_aa_f16v(Pops<__half> a, Geo g, StepK
   const auto as = at.again(g, rows);
   const XLanes xs = FLAT ? XLanes(as, threadIdx.x & 31) : xl;
   const EdgeWarps es = FLAT ? EdgeWarps(as) : ew;
-  int js = FLAT ? as.j : j, ks = k;  // store rows: recomputed after the collision (BGK odd step)
+  int js = FLAT ? as.j : j, ks = k;  // store rows: recomputed after the collision
   asm volatile("" : "+r"(js), "+r"(ks));
   const int jms = js == 0 ? g.ny - 1 : js - 1, jps = js == g.ny - 1 ? 0 : js + 1;
   const int kms = ks == 0 ? g.nz - 1 : ks - 1, kps = ks == g.nz - 1 ? 0 : ks + 1;
