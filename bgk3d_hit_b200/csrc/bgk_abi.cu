@@ -81,7 +81,7 @@ struct bgk_ctx {
   double* partials = nullptr;
   double* h_tot = nullptr;  // pinned: ND totals, zj of the last cell, error flag
   unsigned int* d_max = nullptr;
-  int* d_err = nullptr;     // set on the device when a pipelined kernel's wait ran out
+  int* d_err = nullptr;     // set on the device when a kernel's wait for copies ran out
   int* h_err = nullptr;     // pinned copy
   void* vel = nullptr;
   void* stage = nullptr;
@@ -245,10 +245,10 @@ int set_scale_from_max(bgk_ctx* c) {
 
 int init_layout(const bgk_ctx* c) { return c->scheme == BGK_AA ? LAY_AAE : LAY_TWO; }
 
-// A bounded wait of a pipelined kernel ran out: the step it belonged to did not
+// A kernel's bounded wait for copies ran out: the step it belonged to did not
 // complete.
 int step_failed() {
-  set_err("a stream-collide step gave up waiting for its row copies; populations are invalid");
+  set_err("a stream-collide step gave up waiting for its copies; populations are invalid");
   return BGK_ERR_CUDA;
 }
 
@@ -952,8 +952,9 @@ int bgk_halo_prime(bgk_ctx* c) {
 int bgk_debug_stall_next_step(bgk_ctx* c) {
   int rc = check_ctx(c);
   if (rc) return rc;
-  if (c->p.kernel != 8 || c->p.les_cs > 0.0 || c->slab) {
-    set_err("bgk_debug_stall_next_step needs the row-pipelined kernel (params.kernel = 8, BGK collision)");
+  if (!c->fused && (c->p.kernel != 8 || c->p.les_cs > 0.0 || c->slab)) {
+    set_err("bgk_debug_stall_next_step needs the row-pipelined kernel (params.kernel = 8, BGK collision) or a box "
+            "that takes two steps per launch");
     return BGK_ERR_INVALID;
   }
   c->A.stall = c->B.stall = 1;
@@ -975,6 +976,7 @@ int bgk_run(bgk_ctx* c, int nsteps) {
     for (; s + 2 <= nsteps; s += 2) {
       CK(launch_two_steps(c->A, c->B, c->omega, c->scale, c->p.les_cs, c->st));
       std::swap(c->A, c->B);  // all 19 populations are in b
+      c->A.stall = c->B.stall = 0;
       c->launches++;
       c->step += 2;
     }
@@ -1500,8 +1502,13 @@ int bgk_adjoint(bgk_ctx* c, const double* u0, const double* v0, const double* w0
       if (cur == &work[wi]) wi ^= 1;
       next = &work[wi];
     }
-    if (n == 2) CK(launch_two_steps(*cur, *next, c->omega, 1.0, 0.0, c->st));
-    else CK(launch_step_out_of_place(*cur, *next, c->omega, c->st));
+    if (n == 2) {
+      Lattice src = *cur;
+      std::swap(src.stall, c->A.stall);
+      CK(launch_two_steps(src, *next, c->omega, 1.0, 0.0, c->st));
+    } else {
+      CK(launch_step_out_of_place(*cur, *next, c->omega, c->st));
+    }
     c->launches++;
     cur = next;
     t += n;

@@ -92,6 +92,7 @@ template <class S, int TY> struct Two2 {
     const S* base[Q];
     int yrow[YROWS], yrq[YROWS];  // plane offset of the row that stands for raw row r of population q; q * 64 + r
     unsigned long long bar[2];
+    int failed;  // a wait for a plane ran out
   };
 };
 
@@ -109,7 +110,7 @@ __device__ __forceinline__ int walk_begin(int i, int nz, int lz, int full) {
 template <class F, bool LES, int TY>
 __global__ void __launch_bounds__(Two2<typename F::S, TY>::THREADS, 1)
     k_two2(const __grid_constant__ Two2Maps maps, Pops<const typename F::S> src, Pops<typename F::S> dst, Geo g,
-           StepK K, int lz, int full, int* err) {
+           StepK K, int lz, int full, int* err, int stall) {
   using S = typename F::S;
   using T = Two2<S, TY>;
   constexpr int ROWS = T::ROWS;
@@ -148,6 +149,9 @@ __global__ void __launch_bounds__(Two2<typename F::S, TY>::THREADS, 1)
   };
   auto next = [&](int p) { return p == g.nz - 1 ? 0 : p + 1; };
 
+  // test hook: the first block's first plane is never asked for
+  const bool stalled = stall && (blockIdx.x | blockIdx.y | blockIdx.z) == 0;
+
   // nothing of the step before is read or overwritten before it is done
   step_begin();
 
@@ -156,7 +160,8 @@ __global__ void __launch_bounds__(Two2<typename F::S, TY>::THREADS, 1)
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&sm.bar[1])) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     const int z = modw(z0 - 1, g.nz);
-    issue(0, z);
+    sm.failed = 0;
+    if (!stalled) issue(0, z);
     issue(1, next(z));
   }
   int yn = 0;  // raw rows beyond the y face
@@ -181,14 +186,31 @@ __global__ void __launch_bounds__(Two2<typename F::S, TY>::THREADS, 1)
   // interval k: the first step of plane k beside the second step around plane k - 1
   if (w == T::WORK / 32) {
     int z = next(next(modw(z0 - 1, g.nz)));
-    for (int k = 0; k + 2 < np; ++k, z = next(z)) {
-      // plane k has been read. Two barriers in turn: a warp comes to plane k + 2,
+    // (The form of this loop matters: with its bound at np - 2, or ok preset where the
+    // test hook leaves out plane 0, the same launches are 2-5% slower, us per pair FP64
+    // 256^3 1057 / 1086-1104, FP32 180^3 246 / 246-257.)
+    int asked = 1;  // last plane asked for
+    bool ok = true;
+    for (int k = 0; k < np; ++k, z = next(z)) {
+      if (stalled && k == 0) ok = false;
+      if (k + 2 >= np) continue;
+      // Plane k has been read. Two barriers in turn: a warp comes to plane k + 2,
       // which this warp asks for below, only after this wait is over, but may come
       // to plane k + 1 before this warp comes here, and must not count for plane k
       asm volatile("bar.sync %0, %1;" ::"r"(4 + (k & 1)), "n"(T::ATH + 32) : "memory");
-      if (lane == 0) issue(k, z);
+      // Or it has not come: its copies may still be under way, and its buffer's barrier
+      // is in their phase
+      if (*(volatile int*)&sm.failed) ok = false;
+      if (ok) {
+        if (lane == 0) issue(k, z);
+        asked = k + 2;
+      }
       __syncwarp();
     }
+    // No copy may reach the shared memory of a block that has ended. The first step's
+    // warps have waited for all planes unless one of their waits ran out.
+    for (int k = stalled ? 1 : asked - 1; k <= asked; ++k)
+      (void)mbar_wait(smem_u32(&sm.bar[k & 1]), (k >> 1) & 1, MAX_POLLS);
   } else if (tid < T::ATH) {
     int r, c;  // first-step cell of this thread: row, column of the tile (-1 .. 32)
     if (w < ROWS) {
@@ -227,9 +249,13 @@ __global__ void __launch_bounds__(Two2<typename F::S, TY>::THREADS, 1)
     bool dead = false;
     for (int k = 0; k < np; ++k) {
       S* const raw = &sm.raw[k & 1][0][0];
+      // After a wait that ran out the state is invalid, which is reported; the warp goes
+      // through its remaining intervals on whatever the planes hold.
       if (!mbar_wait(smem_u32(&sm.bar[k & 1]), (k >> 1) & 1, dead ? 1 : MAX_POLLS)) {
-        dead = true;  // reported; the remaining waits are short
+        dead = true;
+        *(volatile int*)&sm.failed = 1;
         *err = 1;
+        __threadfence_block();
       }
       __syncwarp();
       if (yedge) {
@@ -386,7 +412,7 @@ cudaError_t launch(const Lattice& s, const Lattice& d, const StepK& K, cudaStrea
   at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, m, pops<const S>(s), pops<S>(d), g, K, lz, full, s.err);
+  return cudaLaunchKernelEx(&cfg, kern, m, pops<const S>(s), pops<S>(d), g, K, lz, full, s.err, s.stall);
 }
 
 }  // namespace

@@ -17,8 +17,8 @@ struct Lattice {
   int form;
   Geo g;
   void* p[Q];          // population base pointers
-  int* err = nullptr;  // device flag set by a pipelined kernel whose wait ran out
-  int stall = 0;       // test hook: the next pipelined launch waits on a barrier nothing arms
+  int* err = nullptr;  // device flag set by a kernel whose wait for copies ran out
+  int stall = 0;       // test hook: the next launch that waits for copies waits on a barrier nothing arms
 };
 
 // Ghost-plane pointers of a z-slab for one step (see Halo in lattice.cuh):

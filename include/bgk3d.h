@@ -400,11 +400,14 @@ int bgk_diagnostics_noalloc(const void* const* pops19, int lx, int ly, int lz, i
                             double svisc, double omega, double u0, double fp16_scale, int mode, int itime,
                             bgk_diag* out, void* stream);
 
-/* Test hook for the failure path of the row-pipelined kernel (params.kernel
-   = 8): during the next bgk_col_mc its first CTA waits on a barrier that
-   nothing arms; the bounded wait runs out, the step is abandoned and the next
-   synchronising call returns BGK_ERR_CUDA. The context stays usable after a
-   new bgk_init_* or bgk_put_populations. Faults nothing. */
+/* Test hook for the failure path of the kernels that wait for copies: the
+   row-pipelined one (params.kernel = 8) during the next bgk_col_mc, and the one
+   that takes two steps per launch during the next pair of steps of bgk_run or
+   bgk_adjoint. Its first CTA waits on a barrier that nothing arms; the bounded
+   wait runs out, the step is abandoned and the next synchronising call (or
+   bgk_adjoint) returns BGK_ERR_CUDA. The context stays usable after a new
+   bgk_init_* or bgk_put_populations. Faults nothing. BGK_ERR_INVALID for a box
+   that runs neither. */
 int bgk_debug_stall_next_step(bgk_ctx* ctx);
 
 const char* bgk_strerror(int code);
