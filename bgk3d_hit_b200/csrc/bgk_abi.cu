@@ -1105,8 +1105,7 @@ int bgk_get_velocity(bgk_ctx* c, double* u, double* v, double* w) {
     if (piped) CK(cudaEventRecord(c->ev_free[set], sc));
   }
   if (piped) CK(cudaStreamSynchronize(sc));
-  CK(cudaStreamSynchronize(c->st));
-  return BGK_OK;
+  return sync_and_check(c);
 }
 
 int bgk_spectrum(bgk_ctx* c, int nbins, double* ek) {
@@ -1166,8 +1165,7 @@ int bgk_spectrum(bgk_ctx* c, int nbins, double* ek) {
     c->launches++;
   }
   CK(cudaMemcpyAsync(ek, c->d_bins, (size_t)nbins * 8, cudaMemcpyDeviceToHost, c->st));
-  CK(cudaStreamSynchronize(c->st));
-  return BGK_OK;
+  return sync_and_check(c);
 }
 
 // --------------------------------------------------------------- file output
