@@ -83,6 +83,7 @@ struct bgk_ctx {
   unsigned int* d_max = nullptr;
   int* d_err = nullptr;     // set on the device when a kernel's wait for copies ran out
   int* h_err = nullptr;     // pinned copy
+  int* d_adj_err = nullptr; // the same for bgk_adjoint's steps, whose states are its own
   void* vel = nullptr;
   void* stage = nullptr;
   size_t stage_bytes = 0;
@@ -685,9 +686,10 @@ int bgk_create(const bgk_params* p, bgk_ctx** out) {
   if (rc) return fail(rc);
   rc = dev_alloc(c, (void**)&c->d_max, sizeof(unsigned int), "scale probe");
   if (rc) return fail(rc);
-  rc = dev_alloc(c, (void**)&c->d_err, sizeof(int), "error flag");
+  rc = dev_alloc(c, (void**)&c->d_err, 2 * sizeof(int), "error flags");
   if (rc) return fail(rc);
-  e = cudaMemsetAsync(c->d_err, 0, sizeof(int), c->st);
+  c->d_adj_err = c->d_err + 1;
+  e = cudaMemsetAsync(c->d_err, 0, 2 * sizeof(int), c->st);
   if (e != cudaSuccess) return fail(cuda_fail(e, "cudaMemset"));
   e = cudaMallocHost((void**)&c->h_err, sizeof(int));
   if (e != cudaSuccess) return fail(cuda_fail(e, "cudaMallocHost"));
@@ -1352,7 +1354,7 @@ struct AdjBufs {
     void* m = c->lat_pool[next++];
     L->form = c->form;
     L->g = c->g;
-    L->err = c->d_err;
+    L->err = c->d_adj_err;
     for (int q = 0; q < Q; ++q) L->p[q] = (char*)m + (size_t)q * c->g.qs * c->es;
     return BGK_OK;
   }
@@ -1449,6 +1451,7 @@ int bgk_adjoint(bgk_ctx* c, const double* u0, const double* v0, const double* w0
   // when the rounding of K - 1 rebuilt steps grows by at most 64x
   const bool rebuild = want_grad && c->adj_mode == BGK_ADJ_REBUILD && adj_rebuild_ok(c->form, c->omega, K);
   const int nwork = (K - 1 > 2 && !rebuild) ? K - 1 : 2;
+  CK(cudaMemsetAsync(c->d_adj_err, 0, sizeof(int), c->st));
   AdjBufs B(c);
   double *du0 = nullptr, *dut = nullptr, *acc = nullptr, *tot = nullptr;
   if ((rc = upload3(c, 0, u0, v0, w0, &du0, "initial velocity"))) return rc;
@@ -1564,7 +1567,12 @@ int bgk_adjoint(bgk_ctx* c, const double* u0, const double* v0, const double* w0
   }
   double h[2] = {0.0, 0.0};
   CK(cudaMemcpyAsync(h, tot, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->st));
-  if ((rc = sync_and_check(c))) return rc;
+  CK(cudaMemcpyAsync(c->h_err, c->d_adj_err, sizeof(int), cudaMemcpyDeviceToHost, c->st));
+  CK(cudaStreamSynchronize(c->st));
+  if (*c->h_err) {
+    set_err("bgk_adjoint: a step of the forward run gave up waiting for its copies");
+    return BGK_ERR_CUDA;
+  }
   *loss = h[0] / (double)n;
   if (grad_tau) *grad_tau = -c->omega * c->omega * h[1];  // tau = 1/omega
   return BGK_OK;
