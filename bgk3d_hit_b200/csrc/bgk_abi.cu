@@ -73,6 +73,7 @@ struct bgk_ctx {
   size_t es = 8;
   void* memA = nullptr;
   void* memB = nullptr;
+  void* spare = nullptr;  // fused: the second population 19, given back when something else needs it
   Lattice A{}, B{};
   int lay = LAY_TWO;
   int initialized = 0;
@@ -145,8 +146,29 @@ SlabLinks slab_links(const bgk_ctx* c, int rp, int wp) {
 }
 size_t rsize(const bgk_ctx* c) { return c->form == FORM_F64 ? 8 : 4; }
 
+// Gives the second population 19 back: single steps from here, with population 19
+// where they update it in place, in lattice a's block.
+int release_spare(bgk_ctx* c) {
+  const size_t pop = (size_t)c->g.qs * c->es;
+  void* const own = (char*)c->memA + (Q - 1) * pop;
+  if (c->A.p[Q - 1] == c->spare) CK(cudaMemcpyAsync(own, c->spare, pop, cudaMemcpyDeviceToDevice, c->st));
+  CK(cudaStreamSynchronize(c->st));
+  c->A.p[Q - 1] = c->B.p[Q - 1] = own;
+  CK(cudaFree(c->spare));
+  c->spare = nullptr;
+  c->fused = 0;
+  c->dev_bytes -= (long long)pop;
+  return BGK_OK;
+}
+
 int dev_alloc(bgk_ctx* c, void** ptr, size_t bytes, const char* what) {
   cudaError_t e = cudaMalloc(ptr, bytes);
+  if (e == cudaErrorMemoryAllocation && c->spare) {
+    (void)cudaGetLastError();
+    const int rc = release_spare(c);
+    if (rc) return rc;
+    e = cudaMalloc(ptr, bytes);
+  }
   if (e != cudaSuccess) {
     (void)cudaGetLastError();
     *ptr = nullptr;
@@ -669,18 +691,17 @@ int bgk_create(const bgk_params* p, bgk_ctx** out) {
   if (rc) return fail(rc);
   for (int q = 0; q < Q; ++q) c->A.p[q] = (char*)c->memA + q * pop_bytes;
   if (c->scheme == BGK_TWO_LATTICE) {
+    rc = dev_alloc(c, &c->memB, (Q - 1) * pop_bytes, "lattice b");
+    if (rc) return fail(rc);
+    for (int q = 0; q < Q - 1; ++q) c->B.p[q] = (char*)c->memB + q * pop_bytes;
+    c->B.p[Q - 1] = c->A.p[Q - 1];
     // b01..b18, and b19 where two steps run as one: a single step updates pop 19
     // in place (SRC/col_MC.F90:351) and needs no second one. Without the memory
-    // for it the box runs single steps
+    // for it, now or once another allocation fails, the box runs single steps
     c->fused = p->kernel == 0 && !c->slab && p->mode == BGK_CORRECTED &&
-               two_steps_pay(c->g, c->form, p->les_cs > 0.0);
-    if (c->fused && dev_alloc(c, &c->memB, Q * pop_bytes, "lattice b")) c->fused = 0;
-    if (!c->fused) {
-      rc = dev_alloc(c, &c->memB, (Q - 1) * pop_bytes, "lattice b");
-      if (rc) return fail(rc);
-    }
-    for (int q = 0; q < Q - 1; ++q) c->B.p[q] = (char*)c->memB + q * pop_bytes;
-    c->B.p[Q - 1] = c->fused ? (char*)c->memB + (Q - 1) * pop_bytes : c->A.p[Q - 1];
+               two_steps_pay(c->g, c->form, p->les_cs > 0.0) &&
+               dev_alloc(c, &c->spare, pop_bytes, "second population 19") == BGK_OK;
+    if (c->fused) c->B.p[Q - 1] = c->spare;
   }
   rc = dev_alloc(c, (void**)&c->partials, (size_t)DIAG_BLOCKS * ND * 2 * sizeof(double), "diagnostic partials");
   if (rc) return fail(rc);
@@ -723,6 +744,7 @@ int bgk_destroy(bgk_ctx* c) {
   if (c->plan_ok) cufftDestroy(c->plan);
   cudaFree(c->memA);
   cudaFree(c->memB);
+  cudaFree(c->spare);
   cudaFree(c->partials);
   cudaFree(c->d_max);
   cudaFree(c->d_err);
@@ -1135,7 +1157,13 @@ int bgk_spectrum(bgk_ctx* c, int nbins, double* ek) {
     c->fft_bytes = cplx * (dbl ? 16 : 8);
   }
   if (!c->plan_ok) {
-    cufftResult r = cufftPlan3d(&c->plan, nz, ny, nx, dbl ? CUFFT_D2Z : CUFFT_R2C);
+    const cufftType type = dbl ? CUFFT_D2Z : CUFFT_R2C;
+    cufftResult r = cufftPlan3d(&c->plan, nz, ny, nx, type);
+    if (r == CUFFT_ALLOC_FAILED && c->spare) {
+      (void)cudaGetLastError();
+      if ((rc = release_spare(c))) return rc;
+      r = cufftPlan3d(&c->plan, nz, ny, nx, type);
+    }
     if (r != CUFFT_SUCCESS) {
       set_err("cufftPlan3d failed (%d)", (int)r);
       return BGK_ERR_CUDA;

@@ -176,8 +176,9 @@ int bgk_col_mc(bgk_ctx* ctx, int itime);
    the automatic kernel, larger two-lattice boxes in corrected mode (FP64, and FP32
    without the LES collision) take two steps per launch and one pass over the
    populations, with the results of single steps; bgk_create allocates a second
-   population 19 for them (38 arrays instead of 37) and leaves it at single steps
-   where that does not fit the device. */
+   population 19 for them (38 arrays instead of 37), leaves it at single steps where
+   that does not fit the device, and goes back to them, giving the array back, when a
+   later call of the same context finds too little memory. */
 int bgk_run(bgk_ctx* ctx, int nsteps);
 
 /* = diagnostic(itime, icheck, ...) (SRC/diagnostic.F90:25-75): when
