@@ -161,9 +161,10 @@ int release_spare(bgk_ctx* c) {
   return BGK_OK;
 }
 
-int dev_alloc(bgk_ctx* c, void** ptr, size_t bytes, const char* what) {
+// must: the call fails without it, so that the spare array goes first.
+int dev_alloc(bgk_ctx* c, void** ptr, size_t bytes, const char* what, bool must = true) {
   cudaError_t e = cudaMalloc(ptr, bytes);
-  if (e == cudaErrorMemoryAllocation && c->spare) {
+  if (e == cudaErrorMemoryAllocation && must && c->spare) {
     (void)cudaGetLastError();
     const int rc = release_spare(c);
     if (rc) return rc;
@@ -179,7 +180,7 @@ int dev_alloc(bgk_ctx* c, void** ptr, size_t bytes, const char* what) {
   return BGK_OK;
 }
 
-int ensure_stage(bgk_ctx* c, size_t bytes) {
+int ensure_stage(bgk_ctx* c, size_t bytes, bool must = true) {
   if (c->stage_bytes >= bytes) return BGK_OK;
   if (c->stage) {
     CK(cudaStreamSynchronize(c->st));
@@ -188,7 +189,7 @@ int ensure_stage(bgk_ctx* c, size_t bytes) {
     c->stage = nullptr;
     c->stage_bytes = 0;
   }
-  int rc = dev_alloc(c, &c->stage, bytes, "staging buffer");
+  int rc = dev_alloc(c, &c->stage, bytes, "staging buffer", must);
   if (rc) return rc;
   c->stage_bytes = bytes;
   return BGK_OK;
@@ -503,12 +504,16 @@ int copy_direct(bgk_ctx* c, void* out, const void* in, int lay) {
   return out ? sync_and_check(c) : BGK_OK;
 }
 
-// Staging for populations of pop bytes each; *nq: how many it holds at a time.
+// Staging for populations of pop bytes each; *nq: how many it holds at a time, one
+// at least (the size is halved while it cannot be had).
 int ensure_pop_stage(bgk_ctx* c, size_t pop, int* nq) {
   size_t want = (size_t)Q * pop < POP_STAGE_BYTES ? (size_t)Q * pop : POP_STAGE_BYTES;
-  if (want < pop) want = pop;
-  if (want < (size_t)ncell(c) * 8) want = (size_t)ncell(c) * 8;
-  const int rc = ensure_stage(c, want);
+  int rc;
+  for (;; want /= 2) {
+    if (want < pop) want = pop;
+    rc = ensure_stage(c, want, want == pop);
+    if (rc != BGK_ERR_NOMEM || want == pop) break;
+  }
   if (rc) return rc;
   const size_t m = c->stage_bytes / pop;
   *nq = m > (size_t)Q ? Q : (int)m;
@@ -1104,11 +1109,15 @@ int bgk_get_velocity(bgk_ctx* c, double* u, double* v, double* w) {
   if (!u || !v || !w) return BGK_ERR_INVALID;
   CK(cudaSetDevice(c->p.device));
   // chunks of planes through two staging sets: the copies of one chunk run
-  // beside the kernel of the next
-  const int nk = chunk_planes(c);
-  const size_t plane = (size_t)c->g.nx * c->g.ny, chunk = plane * nk;
-  rc = ensure_stage(c, 2 * 3 * chunk * sizeof(double));
+  // beside the kernel of the next; fewer planes where the staging cannot be had
+  const size_t plane = (size_t)c->g.nx * c->g.ny;
+  int nk = chunk_planes(c);
+  for (;; nk = (nk + 1) / 2) {
+    rc = ensure_stage(c, (nk < c->g.nz ? 2 : 1) * 3 * plane * nk * sizeof(double), nk == 1);
+    if (rc != BGK_ERR_NOMEM || nk == 1) break;
+  }
   if (rc) return rc;
+  const size_t chunk = plane * nk;
   const bool piped = nk < c->g.nz;
   if (piped && (rc = begin_transfer(c))) return rc;
   const cudaStream_t sc = piped ? c->st_copy : c->st;
