@@ -1672,6 +1672,8 @@ cudaError_t launch_step_out_of_place(const Lattice& src, const Lattice& dst, dou
       return launch_step(k_two<F64>, sh.grid, sh.block, st, pops_of<const double>(src), pops_of<double>(dst), src.g, K);
     case FORM_F32: {
       const VecRows r(src.g, 2, true);
+      if (!r.pays(src.g, src.g.nz))
+        return launch_step(k_two<F32>, sh.grid, sh.block, st, pops_of<const float>(src), pops_of<float>(dst), src.g, K);
       return launch_vec(k_two_f32v<false, false>, k_two_f32v<false, true>, src.g, r, src.g.nz, st, pops_of<const float>(src),
                  pops_of<float>(dst), src.g, K, r.arg, 0);
     }
@@ -1947,16 +1949,15 @@ static cudaError_t slab_impl(const Lattice& s, const Lattice& d, const StepK& K,
     // kernel (planes 1 .. nz-2 pull only inside the slab, so its z wrap never
     // applies)
     const int ni = s.g.nz - 2;
-    if (F::id == FORM_F32) {
+    const VecRows r(s.g, F::id == FORM_F16 ? 4 : 2, true);
+    if (F::id == FORM_F32 && r.pays(s.g, ni)) {
       Pops<float> pf = pops_of<float>(d);
       pf.p[Q - 1] = (float*)s.p[Q - 1];
-      const VecRows r(s.g, 2, true);
       if (K.les) launch_vec_plain(k_two_f32v<true, false>, k_two_f32v<true, true>, s.g, r, ni, st_in, pops_of<const float>(s), pf, s.g, K, r.arg, 1);
       else launch_vec_plain(k_two_f32v<false, false>, k_two_f32v<false, true>, s.g, r, ni, st_in, pops_of<const float>(s), pf, s.g, K, r.arg, 1);
-    } else if (F::id == FORM_F16) {
+    } else if (F::id == FORM_F16 && r.pays(s.g, ni)) {
       Pops<__half> ph = pops_of<__half>(d);
       ph.p[Q - 1] = (__half*)s.p[Q - 1];
-      const VecRows r(s.g, 4, true);
       if (K.les) launch_vec_plain(k_two_f16v<true, false>, k_two_f16v<true, true>, s.g, r, ni, st_in, pops_of<const __half>(s), ph, s.g, K, r.arg, 1);
       else launch_vec_plain(k_two_f16v<false, false>, k_two_f16v<false, true>, s.g, r, ni, st_in, pops_of<const __half>(s), ph, s.g, K, r.arg, 1);
     } else {

@@ -208,6 +208,13 @@ __device__ __forceinline__ void shift_rows_f32(float2 (&Y)[Q], const float (&E)[
   }
 }
 
+// From how many cells the automatic choice takes the several-cells-per-thread
+// kernels: below, their fewer and longer threads leave the chip idle and one
+// cell per thread is faster. Measured us per step, one cell / several: AA FP16
+// 32^3 4.1 / 5.1, 48^3 6.2 / 7.2, 210,000 cells 7.8 / 8.6, 64^3 7.7 / 7.2; FP32
+// two-lattice 33^3 4.1 / 5.1, 48^3 6.2 / 6.2, 66^3 10.3 / 8.2.
+constexpr long long VEC_MIN_TWO = 1LL << 17, VEC_MIN_AA = 1LL << 18;
+
 // Rows of a V-cells-per-thread kernel: aligned (arg = log2(nx/V)) where nx/V is
 // a power of two and a plane holds whole warps, else flat (arg = chunks of a
 // row). padded: up to a 32-byte sector (8-byte chunks), for kernels that write
@@ -232,14 +239,12 @@ struct VecRows {
     arg = 0;
     while ((1 << arg) < tpr) ++arg;
   }
+  // For the adjoint's steps and the interior of z-slabs (`planes` planes): aligned rows
+  // at any size, others from VEC_MIN_TWO cells. us per step of bgk_adjoint's forward
+  // run, FP32, one cell / two: 33^3 3.6 / 3.7, 40^3 4.15 / 5.0, 45^3 4.3 / 5.1, 50^3 4.2 /
+  // 5.4, 56^3 5.8 / 5.8; two slabs of these sizes on one GPU are bound by the host's
+  // calls (20 us a step either way).
+  bool pays(const Geo& g, int planes) const { return !flat || (long long)g.nx * g.ny * planes >= VEC_MIN_TWO; }
 };
-
-
-// From how many cells the automatic choice takes the several-cells-per-thread
-// kernels: below, their fewer and longer threads leave the chip idle and one
-// cell per thread is faster. Measured us per step, one cell / several: AA FP16
-// 32^3 4.1 / 5.1, 48^3 6.2 / 7.2, 210,000 cells 7.8 / 8.6, 64^3 7.7 / 7.2; FP32
-// two-lattice 33^3 4.1 / 5.1, 48^3 6.2 / 6.2, 66^3 10.3 / 8.2.
-constexpr long long VEC_MIN_TWO = 1LL << 17, VEC_MIN_AA = 1LL << 18;
 
 }  // namespace bgk
