@@ -361,22 +361,39 @@ bool encode(CUtensorMap* m, const Geo& g, int form, void* base, int nq, int cols
 // 1271). FP32: the 1024 threads of a block (TY = 12: 706 us instead of 649).
 template <class F, bool LES> constexpr int tile_rows() { return F::id == FORM_F64 ? (LES ? 6 : 8) : 14; }
 
-// Planes per walk: the sum of all walks (each two planes longer than what it
-// writes) over the SMs, and one walk for the uneven end, in intervals, are least.
-// 256^3 FP64 (256 tiles): 32 planes 998 us, 16 1023, 64 1044.
-struct Walk { int lz; double intervals; };
-Walk best_walk(const Geo& g, int ty, int sms) {
-  const double tiles = (double)((g.nx + TX - 1) / TX) * ((g.ny + ty - 1) / ty);
-  Walk w{g.nz, 1e300};
-  for (int n = 1; n <= g.nz; ++n) {
-    const int lz = (g.nz + n - 1) / n, walks = (g.nz + lz - 1) / lz;
-    const double c = tiles * walks * (lz + 2) / sms + (lz + 2);
-    if (c < w.intervals) w = {lz, c};
-  }
-  return w;
-}
-
 constexpr int SMS = 148;
+
+// How a column of tiles is cut into walks. Planes per walk: the sum of all walks (each
+// two planes longer than what it writes) over the SMs, and one walk for the uneven
+// end, in intervals, are least (256^3 FP64, 256 tiles: 32 planes 998 us, 16 1023, 64
+// 1044). The last walk is halved twice, so that the SMs that are done first are not idle
+// for a whole walk: equal walks / halved, us per two steps of long runs, FP32 256^3 693 /
+// 677, 180^3 271 / 265, 160^3 192 / 189; FP64 256^3 1136 / 1127, 128^3 174.9 / 173.6;
+// Smagorinsky 256^3 1419 / 1418.
+struct Walks {
+  int lz, full, halvings;
+  double tiles;
+  int nz;
+  Walks(const Geo& g, int ty)
+      : lz(g.nz), tiles((double)((g.nx + TX - 1) / TX) * ((g.ny + ty - 1) / ty)), nz(g.nz) {
+    double least = 1e300;
+    for (int n = 1; n <= nz; ++n) {
+      const int l = (nz + n - 1) / n, walks = (nz + l - 1) / l;
+      const double c = tiles * walks * (l + 2) / SMS + (l + 2);
+      if (c < least) {
+        least = c;
+        lz = l;
+      }
+    }
+    full = (nz + lz - 1) / lz - 1;
+    halvings = nz - full * lz >= 4 ? 2 : 0;
+  }
+  int count() const { return full + 1 + halvings; }
+  // Of the whole launch: what all walks take, spread over the SMs, and half a walk for
+  // the end. A walk costs its planes, two more that it does not write, and about half
+  // an interval to start; flat boxes, whose walks are a few planes long, pay the most.
+  double intervals() const { return tiles * (nz + count() * 2.5) / SMS + 0.5 * (lz + 2.5); }
+};
 
 template <class F, bool LES>
 cudaError_t launch(const Lattice& s, const Lattice& d, const StepK& K, cudaStream_t st) {
@@ -395,13 +412,8 @@ cudaError_t launch(const Lattice& s, const Lattice& d, const StepK& K, cudaStrea
       !encode(&m.rest_main, g, s.form, s.p[Q - 1], 1, T::RP, T::ROWS) ||
       !encode(&m.rest_wrap, g, s.form, s.p[Q - 1], 1, T::WP, T::ROWS))
     return cudaErrorInvalidValue;
-  // The last walk is halved twice, so that the SMs that are done first are not idle
-  // for a whole walk. Equal walks / halved, us per two steps of long runs: FP32 256^3
-  // 693 / 677, 180^3 271 / 265, 160^3 192 / 189; FP64 256^3 1136 / 1127, 128^3 174.9 /
-  // 173.6; Smagorinsky 256^3 1419 / 1418.
-  const int lz = best_walk(g, TY, SMS).lz, full = (g.nz + lz - 1) / lz - 1, rest = g.nz - full * lz;
-  const int halvings = rest >= 4 ? 2 : 0;
-  const dim3 grid((g.nx + TX - 1) / TX, (g.ny + TY - 1) / TY, full + 1 + halvings);
+  const Walks w(g, TY);
+  const dim3 grid((g.nx + TX - 1) / TX, (g.ny + TY - 1) / TY, w.count());
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(T::THREADS);
@@ -412,27 +424,34 @@ cudaError_t launch(const Lattice& s, const Lattice& d, const StepK& K, cudaStrea
   at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, m, pops<const S>(s), pops<S>(d), g, K, lz, full, s.err, s.stall);
+  return cudaLaunchKernelEx(&cfg, kern, m, pops<const S>(s), pops<S>(d), g, K, w.lz, w.full, s.err, s.stall);
 }
 
 }  // namespace
 
-// An interval takes about 2.0 us in FP64 and 2.15 in FP32, a single step the time
-// of its cells at the rate given; both sides measured, two steps fused / single in
-// us: FP64 96^3 85 / 90, 112^3 130 / 141, 128^3 165 / 197, 250 x 130 x 130 304 / 395,
-// Smagorinsky 128^3 198 / 201, 180^3 518 / 654, 256^3 1271 / 1533;
-// FP32 256^3 649 / 766, 180^3 266 / 298, 160^3 195 / 199, 128^3 119 / 107. Not built:
-// FP32 Smagorinsky (734 / 757 at 256^3, 306 / 298 at 180^3) and FP16, whose single
-// step (86 GLUPS) is far from bound by memory alone (51 here).
+// An interval of the launch takes about 2.0 us (1.85-2.2 over the boxes below), a
+// single step the time of its cells at the rate given. Runs of 0.7 s, us per two steps,
+// two per launch / single steps:
+//   FP64 80^3 63 / 51, 96^3 78 / 86, 112^3 124 / 139, 128^3 166 / 194, 256^3 1058 / 1524,
+//     250 x 130 x 130 321 / 393, 512 x 512 x 8 224 / 193 and x 16 349 / 385, 1024 x 1024 x
+//     4 645 / 388;
+//   Smagorinsky 112^3 154 / 153, 128^3 198 / 207, 160^3 364 / 468, 256^3 1369 / 1619, 64 x 64 x
+//     512 209 / 207, 512 x 512 x 8 320 / 206 and x 32 788 / 836;
+//   FP32 128^3 107 / 102, 140^3 135 / 148, 160^3 180 / 197, 180^3 251 / 300, 256^3 632 / 770,
+//     1024 x 1024 x 8 499 / 396.
+// Of 97 boxes measured so, the rule takes two that lose 1%, and leaves nine at single
+// steps that would gain 2-8% (one 16%). Not built: FP32 Smagorinsky (734 / 757 at 256^3,
+// 306 / 298 at 180^3, short runs) and FP16, whose single step runs at the copy rate
+// already (86 GLUPS, against 51 and 64 here).
 bool two_steps_pay(const Geo& g, int form, bool les) {
   if (form != FORM_F64 && (form != FORM_F32 || les)) return false;
   const int ty = form == FORM_F64 ? (les ? 6 : 8) : 14;
   // a tile touches one x face and one y face at most; TMA sizes and strides
   if (g.nx < TX + 2 || g.ny < ty + 2) return false;
   const bool aligned = (g.nx & (g.nx - 1)) == 0;
-  const double rate = form == FORM_F64 ? (les ? 20e3 : 21.5e3) : (aligned ? 43.5e3 : 38.5e3);  // cells per us
-  const double us = form == FORM_F64 ? (les ? 2.0 : 2.05) : 2.15;
-  return us * best_walk(g, ty, SMS).intervals < 2.0 * (double)g.nx * g.ny * g.nz / rate;
+  const double rate = form == FORM_F32 ? (aligned ? 43.5e3 : 38.5e3)
+                      : les ? (aligned ? 20e3 : 18.5e3) : (aligned ? 21.5e3 : 20.5e3);  // cells per us
+  return 2.0 * Walks(g, ty).intervals() < 2.0 * (double)g.nx * g.ny * g.nz / rate;
 }
 
 cudaError_t launch_two_steps(const Lattice& src, const Lattice& dst, double omega, double scale, double les_cs,
