@@ -278,11 +278,13 @@ def measured_hbm():
 
 
 def ncu_traffic(kernel_key: str):
+    """DRAM bytes per cell of a launch and the box that was captured, or (None, None)."""
     p = os.path.join(ROOT, "profiles", "ncu_traffic.json")
     try:
-        return json.load(open(p)).get(kernel_key)
+        t = json.load(open(p))
+        return t.get(kernel_key), t["_boxes"].get(kernel_key, "256^3")
     except Exception:
-        return None
+        return None, None
 
 
 def time_steps(box, steps, device):
@@ -315,10 +317,11 @@ def roofline_of(precision, scheme, L, ms_per_step, kernel=0, les=False, launches
     kern = kernel_key(precision, scheme, L, kernel, les)
     if launches_per_step < 1.0:  # two steps per launch (and a single one after an odd count)
         kern = f"k_two2_{precision}" + ("_les" if les else "")
-    tr = ncu_traffic(kern)
+    tr, box = ncu_traffic(kern)
     return {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
             "steps_per_launch": 1.0 / launches_per_step, "traffic": tr * float(L) ** 3 if tr else None, "peak_kind": peak_kind, "bytes_per_cell": bpc,
-            "kernel": kern}
+            "kernel": kern,
+            **({"traffic_note": f"ncu DRAM bytes per cell of the {box} capture x cells"} if tr else {})}
 
 
 def form_line(a, precision, pin, device, fp64_value):
@@ -337,8 +340,6 @@ def form_line(a, precision, pin, device, fp64_value):
         box.close()
     value = float(L) ** 3 * steps / (ms * 1e-3) / 1e9
     rl = roofline_of(precision, "two_lattice", L, ms / steps, launches_per_step=launches / steps)
-    if rl["traffic"] is not None:
-        rl["traffic_note"] = "ncu DRAM bytes per cell of the 256^3 capture x cells"
     return {"value": value, "unit": "GLUPS", "ratio_vs_fp64": value / fp64_value, "steps": steps,
             "warmup": a.warmup, "ms_per_step": ms / steps, "dtype": DTYPE[precision], "scheme": "two_lattice",
             "roofline": rl, "gpu_launches": launches, "clocks": clk}
@@ -368,8 +369,6 @@ def large_line(a, L, precision, scheme, k0, tau, device):
         box.close()
     value = float(L) ** 3 * steps / (ms * 1e-3) / 1e9
     rl = roofline_of(precision, scheme, L, ms / steps, launches_per_step=launches / steps)
-    if rl["traffic"] is not None:
-        rl["traffic_note"] = "ncu DRAM bytes per cell of the 256^3 capture x cells"
     noise = "numpy default_rng" if L ** 3 <= NUMPY_NOISE_MAX_CELLS else "torch CUDA generator"
     return {"workload": f"decaying HIT {L}^3 D3Q19 BGK, {precision} {scheme}, tau={tau}, k0={k0:g}, u_rms=0.03, "
                         f"seed 1234 ({noise} noise)", "box": L, "precision": precision, "scheme": scheme,
@@ -477,8 +476,8 @@ def run_ours(a):
                "d2h_bytes_per_step": diag_bytes * ndiag / a.steps,
                "fixed_ms": fixed, "per_step_ms": per_step,
                "value_at_2000_steps": ws * float(L) ** 3 * 2000 / ((fixed + 2000 * per_step) * 1e-3) / 1e9,
-               "includes": f"velocity upload from pinned host memory and init (fixed_ms), {a.steps} x "
-                           f"(boundaries + col_MC + diagnostic gated by icheck={a.icheck}), diagnostics read back "
+               "includes": f"velocity upload from pinned host memory and init (fixed_ms), {a.steps} steps by "
+                           f"bgk_run up to each diagnostic (every icheck={a.icheck}), diagnostics read back "
                            "(per_step_ms); value_at_2000_steps = the same split at the 2000 steps of the HIT "
                            "256^3 run"}
         box2.close()
@@ -515,6 +514,9 @@ def run_ours(a):
             "config": config_of(a, ws), "roofline": roofline, "cpu_baseline": cpu, "e2e": e2e,
             "gpu_launches": launches, "clocks": clk,
         }
+        if launches < a.steps:  # two steps per launch
+            line["value_note"] = (f"{launches} launches in {ms_max:.1f} ms; in runs of a second the power limit lowers "
+                                  "the clock and two steps per launch settle about a tenth lower (FP64 256^3: 31 GLUPS)")
         if forms is not None:
             line["forms"] = forms
         if large is not None:

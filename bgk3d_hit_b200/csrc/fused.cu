@@ -20,12 +20,13 @@
 // the periodic columns by a second, 32-byte wide box beside the first; rows beyond
 // a y face, which TMA fills with zeros, are put in by the threads.
 //
-// Measured on B200 at 256^3 FP64 (two steps): 985 us, 34 GLUPS (1080-1110 us once the
-// power limit lowers the clock), against 1515 us (22.2, the HBM rate) for two single
-// steps; DRAM 305 bytes a cell for both, FP64 pipe 51% busy, issue slots 47%. What
-// stands between it and the 43 GLUPS of its DRAM bytes is the interval (1.1 us
-// of FP64 pipe, one barrier of all warps per plane). On the way there: both steps
-// by the same warps 25.6 GLUPS (too few warps between barriers), one raw buffer
+// Measured on B200 at 256^3 FP64 (two steps): 944 us, 35.5 GLUPS, over 20 steps at full
+// clock; 1058-1107 us in runs of some tenths of a second, once the power limit lowers
+// the clock; against 1515-1524 us (22.1, the HBM rate) for two single steps. DRAM 305 bytes
+// a cell for both, FP64 pipe 51% busy, issue slots 47%. What stands between it and the
+// 43 GLUPS of its DRAM bytes is the interval (1.1 us of FP64 pipe, one barrier of all
+// warps per plane). Figures of single variants below and at the rules are from the
+// kernel as it stood then, both sides alike. On the way there: both steps by the same warps 25.6 GLUPS (too few warps between barriers), one raw buffer
 // 25.5 (the load of a plane did not fit beside its predecessor's collisions), loads
 // of 8 bytes by cp.async 25.6, the border of all faces patched by the threads
 // 31.2, the boxes issued by a warp that also collides 28.7-31.2, arrive / wait

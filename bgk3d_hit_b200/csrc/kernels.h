@@ -118,7 +118,7 @@ long long faith_planes_elems(const Geo& g);
 cudaError_t launch_faith_snapshot(const Lattice& a, void* out, cudaStream_t st);
 
 // Diagnostics (overlap: launched beside the end of the kernel before, on a
-// context's own stream): per-block partial sums (Neumaier pairs) of ND quantities.
+// context's own stream): per-block partial sums (compensated pairs) of ND quantities.
 // vel (optional, 3*N values of the arithmetic type) receives the local velocity.
 // halo: the ghost planes of a z-slab (in_lo / in_hi), nullptr for a whole box.
 // faith (two-lattice only): pulls that leave the box read the periodic image

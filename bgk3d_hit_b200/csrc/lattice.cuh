@@ -348,8 +348,9 @@ template <class S> struct Pops { S* p[Q]; };
 // Moments and equilibrium deviation in the reference's evaluation order
 // (SRC/col_MC.F90:133-219). x: pulled deviations; e: equilibrium deviations.
 // The reference's cte0 = 0 terms and factors cte1 = 1 are left out (0 + q only
-// turns q = -0 into +0, which rp*(v + q) + s with s >= +0 does not see), and
-// 1/rho is the rounded reciprocal: the same bits with 16 operations less.
+// turns q = -0 into +0, which rp*(v + q) + s does not see: s = rp - p is never -0,
+// as equal operands subtract to +0), and 1/rho is the rounded reciprocal: the same
+// bits with 16 operations less.
 template <class V>
 __device__ __forceinline__ V equilibrium(const V (&x)[Q], V (&e)[Q], V& vxo, V& vyo, V& vzo) {
   using N = Num<V>;

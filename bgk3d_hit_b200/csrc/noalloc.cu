@@ -12,8 +12,8 @@
 // Its only scratch is the file-scope device array below: the per-block
 // compensated partial sums of the diagnostics reduction, a fixed
 // NOALLOC_SCRATCH_BYTES (94,808 bytes) whatever the box size, because the
-// reduction grid is fixed (DIAG_BLOCKS blocks of DIAG_THREADS threads, each
-// thread striding over the cells). Every GPU that loads the library holds this
+// reduction grid depends on the form alone (DIAG_BLOCKS blocks of DIAG_THREADS
+// threads at most, each thread striding over the cells). Every GPU that loads the library holds this
 // array until the process exits.
 #include <cuda_runtime.h>
 
@@ -98,8 +98,10 @@ extern "C" int bgk_diagnostics_noalloc(const void* const* pops19, int lx, int ly
   for (int q = 0; q < Q; ++q) lat.p[q] = const_cast<void*>(pops19[q]);
   cudaStream_t st = (cudaStream_t)stream;
   const bool faithful = mode == BGK_FAITHFUL;
-  // Every partial slot and every total is written by these kernels before it
-  // is read, so nothing left from an earlier call has to be cleared.
+  // Every partial slot that is read, and every total that is used below, is written
+  // by these kernels first, so nothing left from an earlier call has to be cleared
+  // (the enstrophy's total is not computed and not used, that of zj in faithful mode
+  // only).
   cudaError_t e = launch_diag(lat, LAY_TWO, svisc, omega, scale, partials, nullptr, st);
   if (e == cudaSuccess) e = launch_finalize(partials, precision, false, totals, st);
   if (e == cudaSuccess && faithful) e = launch_last_zj(lat, LAY_TWO, scale, totals + ND, st);
